@@ -427,6 +427,7 @@ int create(int nely, int nelx, int nelz, const t3d_params* prm, const t3d_proble
     CHECK(c->alloc(&c->FS, 1));
     CHECK(c->alloc(&c->OC, 1));
     CHECK(c->alloc(&c->scal, 8));
+    if (c->prm.oc_sum_order != T3D_SUM_FP64) CHECK(c->alloc(&c->oc_scratch, (size_t)oc_vec8_bytes(c->ne)));
     double* part = nullptr;
     unsigned int* cnt = nullptr;
     CHECK(c->alloc(&part, 4 * RED_BLOCKS));
@@ -990,14 +991,17 @@ static constexpr int OC_MAX_PASSES = 400;
 
 static int oc_update(Context* c, float V0) {
     const int fp64 = c->prm.oc_sum_order == T3D_SUM_FP64;
-    if (!fp64) CHECK(ensure_morton(c));
     launch_oc_init(c->OC, c->st);
+    if (!fp64) {
+        CHECK(ensure_morton(c));
+        launch_oc_vec8_begin(c->ne, c->morton, c->solid, c->x, c->dc, c->oc_scratch, c->st);
+    }
     int passes = 0;
     for (;;) {
         for (int k = 0; k < 16; ++k) {
-            c->launches += fp64 ? 1 : 2;
-            launch_oc_pass(c->g, c->solid, c->x, c->dc, c->xnew, c->OC, fp64, V0, c->ne, c->slot[0], c->st);
-            if (!fp64) launch_oc_vec8_vol(c->ne, c->morton, c->xnew, c->OC, V0, c->st);
+            c->launches += 1;
+            if (fp64) launch_oc_pass(c->g, c->solid, c->x, c->dc, c->OC, V0, c->ne, c->slot[0], c->st);
+            else launch_oc_vec8_pass(c->ne, c->oc_scratch, c->OC, V0, c->slot[0], c->st);
         }
         CHECK(launch_check("oc pass"));
         passes += 16;
@@ -1006,9 +1010,9 @@ static int oc_update(Context* c, float V0) {
         if (c->flag_h[0]) break;
         if (passes >= OC_MAX_PASSES) return set_error(T3D_ERR_NUMERIC, "OC bisection did not terminate");
     }
-    launch_oc_finish(c->g, c->solid, c->x, c->xnew, c->OC, fp64, c->ne, c->slot[0], c->slot[1], c->st);
-    c->launches += 3 + (fp64 ? 0 : 1);
-    if (!fp64) launch_oc_vec8_stats(c->ne, c->morton, c->x, c->OC, c->st);
+    launch_oc_finish(c->g, c->solid, c->x, c->dc, c->OC, fp64, c->ne, c->slot[0], c->slot[1], c->st);
+    c->launches += 3 + (fp64 ? 0 : 3);
+    if (!fp64) launch_oc_vec8_stats(c->ne, c->morton, c->x, c->oc_scratch, c->OC, c->slot[0], c->st);
     CHECK(launch_check("oc finish"));
     T3D_CUDA_OK(cudaMemcpyAsync(c->OC_h, c->OC, sizeof(OcState), cudaMemcpyDeviceToHost, c->st));
     return sync(c);

@@ -51,6 +51,7 @@ struct Context {
     PcgScalars* S = nullptr;
     FilterScalars* FS = nullptr;
     OcState* OC = nullptr;
+    char* oc_scratch = nullptr; // reference summation order only (oc_vec8_bytes)
     double* scal = nullptr;     // [0] C, [1] Csolid, [2] objective
     bool mv64_stream = false;   // FP64 K(E)u by the element-streaming kernel (else node-centric)
     Stream64Tiling st64{};

@@ -205,23 +205,27 @@ void launch_cells_to_morton_f32(int64_t ne, const int32_t* cell_of, const float*
 // ---- OC (driver.cpp:160-189)
 struct OcState {
     float l1, l2, lmid, vol;
-    float change, sharp, volfrac, pad;
+    float change, sharp, volfrac, rl;   // rl: 2/(l1+l2) of the last pass
     int passes, done, pad1, pad2;
 };
 void launch_dc_scale(const Grid& g, const uint8_t* solid, const float* dcf, const float* x, float* dc,
                      cudaStream_t s);
 void launch_oc_init(OcState* st, cudaStream_t s);
-// one bisection pass: xnew for lmid; fp64_sum: canonical FP64 volume sum + l1/l2 update in the same kernel
-void launch_oc_pass(const Grid& g, const uint8_t* solid, const float* x, const float* dc, float* xnew, OcState* st,
-                    int fp64_sum, float V0, int64_t ne, RedSlot red, cudaStream_t s);
-// reference-order volume sum (8-lane vectorised std::accumulate over Morton order) + l1/l2 update
-void launch_oc_vec8_vol(int64_t ne, const int32_t* morton_cells, const float* xnew, OcState* st, float V0,
-                        cudaStream_t s);
-// change = max|xnew-x|, x = xnew; fp64_sum: sharpness and volume fraction by canonical FP64 sums
-void launch_oc_finish(const Grid& g, const uint8_t* solid, float* x, const float* xnew, OcState* st, int fp64_sum,
+// one bisection pass with the canonical FP64 volume sum
+void launch_oc_pass(const Grid& g, const uint8_t* solid, const float* x, const float* dc, OcState* st, float V0,
+                    int64_t ne, RedSlot red, cudaStream_t s);
+// the same with the reference's float summation order (8-lane vectorised std::accumulate over Morton order):
+// scratch of oc_vec8_bytes(ne) bytes, filled by _begin for one update's densities and sensitivities
+int64_t oc_vec8_bytes(int64_t ne);
+void launch_oc_vec8_begin(int64_t ne, const int32_t* morton_cells, const uint8_t* solid, const float* x,
+                          const float* dc, void* scratch, cudaStream_t s);
+void launch_oc_vec8_pass(int64_t ne, void* scratch, OcState* st, float V0, RedSlot red, cudaStream_t s);
+// x = the last pass's densities, change = their largest step; fp64_sum: sharpness and volume fraction by
+// canonical FP64 sums
+void launch_oc_finish(const Grid& g, const uint8_t* solid, float* x, const float* dc, OcState* st, int fp64_sum,
                       int64_t ne, RedSlot r1, RedSlot r2, cudaStream_t s);
-// reference-order sharpness and volume fraction
-void launch_oc_vec8_stats(int64_t ne, const int32_t* morton_cells, const float* x, OcState* st, cudaStream_t s);
+void launch_oc_vec8_stats(int64_t ne, const int32_t* morton_cells, const float* x, void* scratch, OcState* st,
+                          RedSlot red, cudaStream_t s);
 
 // ---- mixed precision (k_mixed.cu)
 // FP64 node vector (3 planes, rows of nnx) -> FP32 image (rows of px, pads zero), and back
