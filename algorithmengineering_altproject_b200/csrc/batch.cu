@@ -68,8 +68,8 @@ struct Batch {
     ModalKe kh{};
     std::vector<void*> dallocs;
     bool standard = false;       // the members' V-cycle (all the same): Standard, else Adapted
-    LaunchList mv, up, dir, p0, co, mv1, mv2;
-    LaunchList rs0[8], rs1[8], pr[8], lop[8], lmv[8], pa[8];
+    LaunchList mv, up, dir, p0, co, mv1, mv2, jac;
+    LaunchList rs0[8], rs1[8], pr[8], lop[8], pa[8];
     int maxL = 0, coarse_max = 0;
     CUtensorMap* maps = nullptr;
     std::vector<BatchCompact> compact;   // one compaction job per launch list
@@ -124,8 +124,8 @@ struct Batch {
         dS = nullptr;
         dflags = nullptr;
         err = nullptr;
-        mv = up = dir = p0 = co = mv1 = mv2 = LaunchList{};
-        for (int l = 0; l < 8; ++l) rs0[l] = rs1[l] = pr[l] = lop[l] = lmv[l] = pa[l] = LaunchList{};
+        mv = up = dir = p0 = co = mv1 = mv2 = jac = LaunchList{};
+        for (int l = 0; l < 8; ++l) rs0[l] = rs1[l] = pr[l] = lop[l] = pa[l] = LaunchList{};
     }
 
     ~Batch() {
@@ -268,7 +268,10 @@ static int batch_lists(Batch* B) {
         auto below = [l](const t3d_context* c) { return c->nlev - 1 > l; };
         auto rs = [&, l](t3d_context* c, int) {
             const float* src = B->standard ? (l == 0 ? c->Ap32 : c->vtmp32[l]) : (l == 0 ? c->r32 : c->lv32[l].r);
-            return BatchRestrict{c->lv32[l + 1], c->lv32[l], src, c->ra1_32[l], c->lv32[l + 1].r, c->S32, norm};
+            // the Standard cycle starts the coarse level in the same kernel (the coarsest level is solved instead)
+            float* x0 = B->standard && l + 2 < c->nlev ? c->lv32[l + 1].x : nullptr;
+            return BatchRestrict{c->lv32[l + 1], c->lv32[l], src, c->ra1_32[l], c->lv32[l + 1].r, c->S32, norm, x0,
+                                 c->prm.mg_standard_weight};
         };
         CHECK(list(&B->rs0[l], below, rs, [](const BatchRestrict& a) { return batch_blocks_restrict(a, 0); }));
         CHECK(list(&B->rs1[l], [&, l](const t3d_context* c) {
@@ -281,25 +284,27 @@ static int batch_lists(Batch* B) {
                 }, [](const BatchProlong& a) { return batch_blocks_prolong(a); }));
             continue;
         }
-        // the Standard cycle's level steps, level matrices and prolongations (level 0: z, r and the TMA products)
-        CHECK(list(&B->lop[l], below, [l](t3d_context* c, int) {
-            const MgLevel32& L = c->lv32[l];
-            return l == 0 ? BatchLevelOp{L, c->r32, nullptr, c->z32, c->prm.mg_standard_weight, c->S32}
-                          : BatchLevelOp{L, L.r, c->vtmp32[l], L.x, c->prm.mg_standard_weight, c->S32};
-        }, [](const BatchLevelOp& a) { return batch_blocks_level_op(a); }));
+        // the Standard cycle's prolongations and level products; a level's corrected x is in its vtmp32
         CHECK(list(&B->pa[l], below, [l](t3d_context* c, int) {
             const MgLevel32 &Lc = c->lv32[l + 1], &Lf = c->lv32[l];
-            return l == 0 ? BatchProlongAdd{Lc, Lf, Lc.x, c->z32, c->Ap32, c->S32}
-                          : BatchProlongAdd{Lc, Lf, Lc.x, Lf.x, Lf.x, c->S32};
+            const float* xc = l + 2 < c->nlev ? c->vtmp32[l + 1] : Lc.x;
+            return l == 0 ? BatchProlongAdd{Lc, Lf, xc, c->z32, c->Ap32, c->S32}
+                          : BatchProlongAdd{Lc, Lf, xc, Lf.x, Lf.x, c->S32};
         }, [](const BatchProlongAdd& a) { return batch_blocks_prolong_add(a); }));
         if (l >= 1) {
-            CHECK(list(&B->lmv[l], below, [l](t3d_context* c, int) {
-                return BatchLevelMatvec{c->lv32[l], c->Kel32[l], c->lv32[l].x, c->vtmp32[l], c->S32};
-            }, [](const BatchLevelMatvec& a) { return batch_blocks_level_matvec(a); }));
-            // each level op and level product runs twice per cycle (down and up)
-            B->iter_kernels += 2;
-            B->iter_blocks += B->lop[l].blocks + B->lmv[l].blocks;
+            CHECK(list(&B->lop[l], below, [l](t3d_context* c, int) {
+                const MgLevel32& L = c->lv32[l];
+                return BatchLevelOp{L, c->Kel32[l], L.x, L.r, c->vtmp32[l], c->prm.mg_standard_weight, c->S32};
+            }, [](const BatchLevelOp& a) { return batch_blocks_level_op(a); }));
+            // each level product runs twice per cycle (down and up)
+            B->iter_kernels += 1;
+            B->iter_blocks += B->lop[l].blocks;
         }
+    }
+    if (B->standard) {
+        CHECK(list(&B->jac, all, [](t3d_context* c, int) {
+            return BatchJacobi{c->lv32[0], c->r32, c->z32, c->prm.mg_standard_weight, c->S32};
+        }, [](const BatchJacobi& a) { return batch_blocks_jacobi(a); }));
     }
     if (B->standard) {
         CHECK(list(&B->mv1, all, [&](t3d_context* c, int i) {
@@ -406,24 +411,19 @@ static void batch_vcycle(Batch* B) {
         launch_batch_prolong0_32(args_of<BatchProlong0>(B->p0), B->p0.act, B->p0.n, B->st);
         return;
     }
+    launch_batch_jacobi32(args_of<BatchJacobi>(B->jac), B->jac.act, B->jac.n, B->st);        // z = w r / D
     for (int l = 0; l + 1 < B->maxL; ++l) {
         const LaunchList& op = B->lop[l];
-        launch_batch_level_op32(args_of<BatchLevelOp>(op), op.act, op.n, 0, B->st);          // x = w r / D
-        if (l == 0) {
-            batch_product(B, 1, B->mv1);                                                     // t = r - K x
-        } else {
-            const LaunchList& mv = B->lmv[l];
-            launch_batch_level_matvec32(args_of<BatchLevelMatvec>(mv), mv.act, mv.n, B->st);   // t = K x
-            launch_batch_level_op32(args_of<BatchLevelOp>(op), op.act, op.n, 1, B->st);      // t = r - t
-        }
-        batch_restrict(B, l);                                                                // r' = P^T t
+        if (l == 0) batch_product(B, 1, B->mv1);                                                     // t = r - K x
+        else if (op.n) launch_batch_level_op32(args_of<BatchLevelOp>(op), op.act, op.n, false, B->st);
+        batch_restrict(B, l);                                          // r' = P^T t, x' = w r' / D'
     }
     launch_batch_coarse32(args_of<BatchCoarse>(B->co), B->co.act, B->co.n, B->coarse_max, B->st);
     for (int l = B->maxL - 2; l >= 1; --l) {
-        const LaunchList &pa = B->pa[l], &mv = B->lmv[l], &op = B->lop[l];
-        launch_batch_prolong_add32(args_of<BatchProlongAdd>(pa), pa.act, pa.n, B->st);       // x += P x'
-        launch_batch_level_matvec32(args_of<BatchLevelMatvec>(mv), mv.act, mv.n, B->st);     // t = K x
-        launch_batch_level_op32(args_of<BatchLevelOp>(op), op.act, op.n, 2, B->st);          // x += w (r - t) / D
+        const LaunchList &pa = B->pa[l], &op = B->lop[l];
+        if (!pa.n) continue;
+        launch_batch_prolong_add32(args_of<BatchProlongAdd>(pa), pa.act, pa.n, B->st);        // x += P x'
+        launch_batch_level_op32(args_of<BatchLevelOp>(op), op.act, op.n, true, B->st);        // t = x + w (r - K x) / D
     }
     launch_batch_prolong_add32(args_of<BatchProlongAdd>(B->pa[0]), B->pa[0].act, B->pa[0].n, B->st);   // T = z + P x'
     batch_product(B, 2, B->mv2);                                      // z = T + w (r - K T) / D, with r.z

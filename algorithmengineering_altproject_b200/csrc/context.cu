@@ -661,45 +661,40 @@ int matvec64(Context* c, const double* u, double* y, RedSlot dot, PcgScalars* S)
     return 2;
 }
 
-// y = K_l x on level l (level 0: K(E) of the moduli the hierarchy was built from)
-static void level_matvec(Context* c, int l, const double* x, double* y, const PcgScalars* S) {
-    if (l == 0)
-        launch_matvec64_stream(c->g, c->st64, c->Ke_h, c->ke_pat ? c->Kd : nullptr, c->E_mg, c->mask0, x, y, S,
-                               c->st);
-    else
-        launch_level_matvec(c->lv[l], c->KelT[l], x, y, S, c->st);
-}
-
 // kernels of one V-cycle
 static int vcycle_launches(const Context* c) {
     const int L = c->nlev;
-    return c->standard ? 9 * (L - 1) + 2 : 4 * (L - 1) + 1;
+    return c->standard ? 6 * (L - 1) + 5 : 4 * (L - 1) + 1;
 }
 
 // The 'Standard' cycle (see k_mg_standard.cu); level 0 uses Ap as scratch (free between the PCG update
-// and the next K(E)p)
+// and the next K(E)p), and the moduli the hierarchy was built from.  On the coarse levels the residual and the
+// correction are part of the level product, the start part of the restriction; the corrected x goes to vtmp.
 static void vcycle_standard(Context* c, const double* r, double* z, PcgScalars* S, RedSlot dot) {
     const int L = c->nlev;
     const double w = (double)c->prm.mg_standard_weight;
+    const double* Kd = c->ke_pat ? c->Kd : nullptr;
     c->launches += vcycle_launches(c);
+    launch_jacobi_init(c->lv[0], r, z, w, S, c->st);
+    launch_matvec64_stream(c->g, c->st64, c->Ke_h, Kd, c->E_mg, c->mask0, z, c->Ap, S, c->st);
+    launch_residual(c->lv[0], r, c->Ap, S, c->st);
     for (int l = 0; l + 1 < L; ++l) {
-        const double* rl = l == 0 ? r : c->lv[l].r;
-        double* xl = l == 0 ? z : c->lv[l].x;
-        double* t = l == 0 ? c->Ap : c->vtmp[l];
-        launch_jacobi_init(c->lv[l], rl, xl, w, S, c->st);
-        level_matvec(c, l, xl, t, S);
-        launch_residual(c->lv[l], rl, t, S, c->st);
-        launch_restrict(c->lv[l + 1], c->lv[l], t, c->lv[l + 1].r, c->ra1[l], c->ra2[l], S, c->st, false);
+        const MgLevel &Lf = c->lv[l], &Lc = c->lv[l + 1];
+        if (l > 0) launch_level_op(Lf, c->KelT[l], Lf.x, Lf.r, c->vtmp[l], false, w, S, c->st);
+        launch_restrict(Lc, Lf, l == 0 ? c->Ap : c->vtmp[l], Lc.r, c->ra1[l], c->ra2[l], S, c->st, false,
+                        l + 2 < L ? Lc.x : nullptr, w);
     }
     launch_coarse_solve(c->lv[L - 1], c->Xc, c->Nc, c->chol_status, S, c->st);
-    for (int l = L - 2; l >= 0; --l) {
-        const double* rl = l == 0 ? r : c->lv[l].r;
-        double* xl = l == 0 ? z : c->lv[l].x;
-        double* t = l == 0 ? c->Ap : c->vtmp[l];
-        launch_prolong_add(c->lv[l + 1], c->lv[l], c->lv[l + 1].x, xl, S, c->st);
-        level_matvec(c, l, xl, t, S);
-        launch_jacobi_correct(c->lv[l], rl, t, xl, w, S, c->st);
+    const double* xc = c->lv[L - 1].x;
+    for (int l = L - 2; l >= 1; --l) {
+        const MgLevel& Lf = c->lv[l];
+        launch_prolong_add(c->lv[l + 1], Lf, xc, Lf.x, S, c->st);
+        launch_level_op(Lf, c->KelT[l], Lf.x, Lf.r, c->vtmp[l], true, w, S, c->st);
+        xc = c->vtmp[l];
     }
+    launch_prolong_add(c->lv[1], c->lv[0], xc, z, S, c->st);
+    launch_matvec64_stream(c->g, c->st64, c->Ke_h, Kd, c->E_mg, c->mask0, z, c->Ap, S, c->st);
+    launch_jacobi_correct(c->lv[0], r, c->Ap, z, w, S, c->st);
     if (S) launch_dot_rz(c->g.NN, r, z, dot, S, c->st);
 }
 
@@ -789,51 +784,47 @@ static void vcycle32_standard(Context* c, const float* r, float* z, PcgScalars* 
     const float w = c->prm.mg_standard_weight;
     // level 0 with the modal TMA kernel: the residual and the correction (with r.z) run in its epilogue
     const bool fuse = c->modal && modal_fused_available(c->mt);
-    auto level_op = [&](int l, const float* x, float* y) {
-        if (l == 0) matvec32(c, x, y, RedSlot{nullptr, nullptr}, S, 0, c->E_mg32);
-        else {
-            launch_level_matvec32(c->lv32[l], c->Kel32[l], x, y, S, c->st);
-            c->launches += 1;
-        }
+    auto product0 = [&](const float* x, float* y) {
+        matvec32(c, x, y, RedSlot{nullptr, nullptr}, S, 0, c->E_mg32);
     };
+    launch_jacobi_init32(c->lv32[0], r, z, w, S, c->st);
+    c->launches += 2;
+    if (fuse) {
+        launch_matvec32_fused(1, c->g, c->kh, c->mt, c->E_mg32, c->mask0, z, c->Ap32, r, nullptr, w,
+                              RedSlot{nullptr, nullptr}, S, c->tma_err, c->st);
+    } else {
+        product0(z, c->Ap32);
+        launch_residual32(c->lv32[0], r, c->Ap32, S, c->st);
+    }
+    // coarse levels: the residual and the correction are part of the level product, the start part of the
+    // restriction; a level's corrected x is in vtmp32
     for (int l = 0; l + 1 < L; ++l) {
-        const float* rl = l == 0 ? r : c->lv32[l].r;
-        float* xl = l == 0 ? z : c->lv32[l].x;
-        float* t = l == 0 ? c->Ap32 : c->vtmp32[l];
-        launch_jacobi_init32(c->lv32[l], rl, xl, w, S, c->st);
-        c->launches += 1;
-        if (l == 0 && fuse) {
-            launch_matvec32_fused(1, c->g, c->kh, c->mt, c->E_mg32, c->mask0, xl, t, rl, nullptr, w,
-                                  RedSlot{nullptr, nullptr}, S, c->tma_err, c->st);
-            c->launches += 1;
-        } else {
-            level_op(l, xl, t);
-            launch_residual32(c->lv32[l], rl, t, S, c->st);
-            c->launches += 1;
-        }
-        launch_restrict32(c->lv32[l + 1], c->lv32[l], t, c->lv32[l + 1].r, c->ra1_32[l], S, c->st, false);
-        c->launches += c->lv32[l + 1].span == 4 ? 2 : 1;
+        const MgLevel32 &Lf = c->lv32[l], &Lc = c->lv32[l + 1];
+        if (l > 0) launch_level_op32(Lf, c->Kel32[l], Lf.x, Lf.r, c->vtmp32[l], false, w, S, c->st);
+        launch_restrict32(Lc, Lf, l == 0 ? c->Ap32 : c->vtmp32[l], Lc.r, c->ra1_32[l], S, c->st, false,
+                          l + 2 < L ? Lc.x : nullptr, w);
+        c->launches += (l > 0) + (Lc.span == 4 ? 2 : 1);
     }
     launch_coarse_solve32(c->lv32[L - 1], c->Xc, c->Nc, c->chol_status, S, c->st);
     c->launches += 1;
+    const float* xc = c->lv32[L - 1].x;
     for (int l = L - 2; l >= 1; --l) {
-        const float* rl = c->lv32[l].r;
-        float* xl = c->lv32[l].x;
-        launch_prolong_add32(c->lv32[l + 1], c->lv32[l], c->lv32[l + 1].x, xl, xl, S, c->st);
-        level_op(l, xl, c->vtmp32[l]);
-        launch_jacobi_correct32(c->lv32[l], rl, c->vtmp32[l], xl, w, S, c->st);
+        const MgLevel32& Lf = c->lv32[l];
+        launch_prolong_add32(c->lv32[l + 1], Lf, xc, Lf.x, Lf.x, S, c->st);
+        launch_level_op32(Lf, c->Kel32[l], Lf.x, Lf.r, c->vtmp32[l], true, w, S, c->st);
+        xc = c->vtmp32[l];
         c->launches += 2;
     }
     // level 0: T = z + P x_1 into Ap32, then z = T + w (r - K T) / D with r.z, fused; else the separate steps
     if (fuse) {
-        launch_prolong_add32(c->lv32[1], c->lv32[0], c->lv32[1].x, z, c->Ap32, S, c->st);
+        launch_prolong_add32(c->lv32[1], c->lv32[0], xc, z, c->Ap32, S, c->st);
         launch_matvec32_fused(2, c->g, c->kh, c->mt, c->E_mg32, c->mask0, c->Ap32, z, r, c->lv32[0].diag, w, dot, S,
                               c->tma_err, c->st);
         c->launches += 2;
         return;
     }
-    launch_prolong_add32(c->lv32[1], c->lv32[0], c->lv32[1].x, z, z, S, c->st);
-    level_op(0, z, c->Ap32);
+    launch_prolong_add32(c->lv32[1], c->lv32[0], xc, z, z, S, c->st);
+    product0(z, c->Ap32);
     launch_jacobi_correct32(c->lv32[0], r, c->Ap32, z, w, S, c->st);
     launch_dot_rz32(3 * c->g.NNp, r, z, dot, S, c->st);
     c->launches += 3;

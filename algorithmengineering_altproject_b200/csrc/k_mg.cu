@@ -170,7 +170,7 @@ __global__ void k_restrict_y(MgLevel Lc, MgLevel Lf, const double* __restrict__ 
 // normalize = 0: the plain hat-weighted sum, i.e. the transpose of the trilinear prolongation (the
 // 'Standard' V-cycle option)
 __global__ void k_restrict_z(MgLevel Lc, MgLevel Lf, const double* __restrict__ a2, double* __restrict__ rc,
-                             const PcgScalars* S, int normalize) {
+                             const PcgScalars* S, int normalize, double* __restrict__ x0, double w0) {
     if (S != nullptr && S->done) return;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= Lc.nn) return;
@@ -209,9 +209,15 @@ __global__ void k_restrict_z(MgLevel Lc, MgLevel Lf, const double* __restrict__ 
         o2 = v2 * iw;
     }
     const int m = Lc.mask[n];
-    rc[n] = (m & 1) ? 0.0 : o0;
-    rc[Lc.nn + n] = (m & 2) ? 0.0 : o1;
-    rc[2 * Lc.nn + n] = (m & 4) ? 0.0 : o2;
+    const double o[3] = {(m & 1) ? 0.0 : o0, (m & 2) ? 0.0 : o1, (m & 4) ? 0.0 : o2};
+    for (int c = 0; c < 3; ++c) {
+        const int64_t i = c * Lc.nn + n;
+        rc[i] = o[c];
+        if (x0) {   // the Standard cycle's Jacobi start x0 = w0 rc / D
+            const double d = Lc.diag[i];
+            x0[i] = ((m >> c) & 1) ? 0.0 : (w0 * o[c]) * (1.0 / (1.0e-30 < d ? d : 1.0e-30));
+        }
+    }
 }
 
 // coarsest Jacobi fallback x = r/max(1e-30,D) without weight, masked (preconditioner.cpp:199-227)
@@ -573,12 +579,12 @@ void launch_diag_coarsen(const MgLevel& Lc, const MgLevel& Lf, cudaStream_t s) {
     k_diag_coarsen<<<blocks_for(Lc.nn, 128), 128, 0, s>>>(Lc, Lf);
 }
 void launch_restrict(const MgLevel& Lc, const MgLevel& Lf, const double* rf, double* rc, double* a1, double* a2,
-                     const PcgScalars* S, cudaStream_t s, bool normalize) {
+                     const PcgScalars* S, cudaStream_t s, bool normalize, double* x0, double w) {
     const int64_t n1 = (int64_t)(Lf.nz + 1) * (Lf.ny + 1) * (Lc.nx + 1);
     const int64_t n2 = (int64_t)(Lf.nz + 1) * (Lc.ny + 1) * (Lc.nx + 1);
     k_restrict_x<<<blocks_for(n1, 256), 256, 0, s>>>(Lc, Lf, rf, a1, S);
     k_restrict_y<<<blocks_for(n2, 256), 256, 0, s>>>(Lc, Lf, a1, a2, S);
-    k_restrict_z<<<blocks_for(Lc.nn, 128), 128, 0, s>>>(Lc, Lf, a2, rc, S, normalize ? 1 : 0);
+    k_restrict_z<<<blocks_for(Lc.nn, 128), 128, 0, s>>>(Lc, Lf, a2, rc, S, normalize ? 1 : 0, x0, w);
 }
 void launch_coarse_jacobi(const MgLevel& L, const PcgScalars* S, cudaStream_t s) {
     k_coarse_jacobi<<<blocks_for(L.nn, 128), 128, 0, s>>>(L, S);

@@ -15,6 +15,7 @@
 // read an entry-major copy (kel_index: entry k of element e at k * ne + e), in which threads working on
 // consecutive nodes read consecutive addresses.
 #include "kernels.hpp"
+#include "level_product.cuh"
 #include "red.cuh"
 
 namespace t3d {
@@ -250,39 +251,52 @@ __global__ void k_level_diag(MgLevel L, const double* __restrict__ Kel) {
     }
 }
 
-// y = K_l x from the entry-major element matrices KelT (node-centric gather), fixed DOFs 0
-__global__ void k_level_matvec(MgLevel L, const double* __restrict__ Kel, const double* __restrict__ x,
-                               double* __restrict__ y, const PcgScalars* S) {
-    if (S != nullptr && S->done) return;
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= L.nn) return;
-    const int nnx = L.nx + 1, nny = L.ny + 1;
-    const int X = n % nnx, Y = (n / nnx) % nny, Z = n / (nnx * nny);
-    const int64_t ne = (int64_t)L.nx * L.ny * L.nz;
-    double acc[3] = {0.0, 0.0, 0.0};
-    for (int dz = 0; dz <= 1; ++dz)
-        for (int dy = 0; dy <= 1; ++dy)
-            for (int dx = 0; dx <= 1; ++dx) {
-                const int ex = X - dx, ey = Y - dy, ez = Z - dz;
-                if (ex < 0 || ey < 0 || ez < 0 || ex >= L.nx || ey >= L.ny || ez >= L.nz) continue;
-                const int a = corner_of(dx, dy, dz);
-                const double* K = Kel + ((ez * L.ny + ey) * L.nx + ex);   // entry k at K[k * ne]
-                for (int b = 0; b < 8; ++b) {
-                    const int m = lnode(L, ex + corner_dx(b), ey + corner_dy(b), ez + corner_dz(b));
-                    for (int c = 0; c < 3; ++c) {
-                        const double xv = x[c * L.nn + m];
-                        for (int r = 0; r < 3; ++r) acc[r] = acc[r] + K[((3 * a + r) * 24 + 3 * b + c) * ne] * xv;
-                    }
-                }
-            }
-    const int mk = L.mask[n];
-    for (int r = 0; r < 3; ++r) y[r * L.nn + n] = ((mk >> r) & 1) ? 0.0 : acc[r];
-}
-
 __device__ __forceinline__ double inv_diag(const MgLevel& L, int c, int n) {
     const double d = L.diag[c * L.nn + n];
     return 1.0 / (1.0e-30 < d ? d : 1.0e-30);
 }
+
+// y = r - K_l x or y = x + w (r - K_l x) / D (y other than x) from the entry-major element matrices, fixed DOFs 0
+template <LevelOp OP>
+__device__ __forceinline__ void level_store(const MgLevel& L, int n, int row, double kx, const double* __restrict__ x,
+                                            const double* __restrict__ r, double* __restrict__ y, double w) {
+    const bool fixed = (L.mask[n] >> row) & 1;
+    const int64_t i = row * L.nn + n;
+    if (OP == LevelOp::Residual) y[i] = fixed ? 0.0 : r[i] - kx;
+    else y[i] = fixed ? 0.0 : x[i] + (w * (r[i] - kx)) * inv_diag(L, row, n);
+}
+struct FullRow {   // the 24 entries of a row of the entry-major matrices
+    int ne;
+    template <class F>
+    __device__ __forceinline__ void operator()(int i, F&& take) const {
+#pragma unroll
+        for (int j = 0; j < 24; ++j) take(j, (int64_t)(24 * i + j) * ne);
+    }
+};
+template <LevelOp OP>
+__global__ void __launch_bounds__(LS_THREADS, 1) k_level_split(MgLevel L, const double* __restrict__ Kel,
+                                                               const double* __restrict__ x,
+                                                               const double* __restrict__ r, double* __restrict__ y,
+                                                               double w, const PcgScalars* S) {
+    __shared__ double sums[3 * LS_NODES];
+    if (S != nullptr && S->done) return;
+    level_split<double>(L, L.nn, (int64_t)blockIdx.x * LS_NODES, Kel, x, sums, FullRow{L.nx * L.ny * L.nz},
+                        [&](int n, int row, double kx) { level_store<OP>(L, n, row, kx, x, r, y, w); });
+}
+template <LevelOp OP>
+__global__ void __launch_bounds__(96, 5) k_level_nodes(MgLevel L, const double* __restrict__ Kel,
+                                                       const double* __restrict__ x, const double* __restrict__ r,
+                                                       double* __restrict__ y, double w, const PcgScalars* S) {
+    if (S != nullptr && S->done) return;
+    const int n = blockIdx.x * 32 + (threadIdx.x & 31), row = threadIdx.x >> 5;
+    if (n >= L.nn) return;
+    double kx[1];
+    level_nodes<1, double>(L, L.nn, n, row, Kel, x, FullRow{L.nx * L.ny * L.nz}, kx);
+    level_store<OP>(L, n, row, kx[0], x, r, y, w);
+}
+// nodes up to which the split form is used: four waves of its blocks (one per SM).  At 30,625 nodes a V-cycle at
+// 96x192x96 takes 0.764 ms split, 0.731 not.
+constexpr int64_t LEVEL_SPLIT_MAX = 4 * 148 * LS_NODES;
 
 // x = w r / D
 __global__ void k_jacobi_init(MgLevel L, const double* __restrict__ r, double* __restrict__ x, double w,
@@ -443,9 +457,17 @@ void launch_galerkin_coarse(const MgLevel& Lf, const MgLevel& Lc, const double* 
 void launch_level_diag(const MgLevel& L, const double* Kel, cudaStream_t s) {
     k_level_diag<<<blocks_of(L.nn, 256), 256, 0, s>>>(L, Kel);
 }
-void launch_level_matvec(const MgLevel& L, const double* Kel, const double* x, double* y, const PcgScalars* S,
-                         cudaStream_t s) {
-    k_level_matvec<<<blocks_of(L.nn, 128), 128, 0, s>>>(L, Kel, x, y, S);
+void launch_level_op(const MgLevel& L, const double* Kel, const double* x, const double* r, double* y, bool correct,
+                     double w, const PcgScalars* S, cudaStream_t s) {
+    const unsigned b = blocks_of(L.nn, 32);
+    static_assert(LS_NODES == 32, "both forms take 32 nodes a block");
+    if (L.nn <= LEVEL_SPLIT_MAX) {
+        if (correct) k_level_split<LevelOp::Correct><<<b, LS_THREADS, 0, s>>>(L, Kel, x, r, y, w, S);
+        else k_level_split<LevelOp::Residual><<<b, LS_THREADS, 0, s>>>(L, Kel, x, r, y, w, S);
+        return;
+    }
+    if (correct) k_level_nodes<LevelOp::Correct><<<b, 96, 0, s>>>(L, Kel, x, r, y, w, S);
+    else k_level_nodes<LevelOp::Residual><<<b, 96, 0, s>>>(L, Kel, x, r, y, w, S);
 }
 void launch_jacobi_init(const MgLevel& L, const double* r, double* x, double w, const PcgScalars* S, cudaStream_t s) {
     k_jacobi_init<<<blocks_of(L.nn, 256), 256, 0, s>>>(L, r, x, w, S);

@@ -12,6 +12,7 @@
 #include <type_traits>
 
 #include "kernels.hpp"
+#include "level_product.cuh"
 #include "red.cuh"
 
 namespace t3d {
@@ -250,51 +251,76 @@ __host__ __device__ constexpr int sym_pack(int i, int j) {
 }
 constexpr int SYM_N = 300;
 
-// y = K_l x from the FP32 element matrices of a coarse level, stored symmetric-packed and entry-major (entry p of
-// element e at p * ne + e; the Galerkin operators P^T K P are symmetric).  Node-centric gather: each node reads
-// the three rows of its corner in the 8 element matrices around it (all loops unrolled, so the packed positions
-// are constants); consecutive nodes read consecutive addresses.  Fixed DOFs 0.
-__device__ __forceinline__ void level_matvec32(VB vb, const MgLevel32& L, const float* __restrict__ Kel,
-                                               const float* __restrict__ x, float* __restrict__ y,
-                                               const PcgScalars* S) {
-    if (S->done) return;
-    const int nnx = L.nx + 1, nny = L.ny + 1;
-    const int64_t ne = (int64_t)L.nx * L.ny * L.nz;
-    for (int64_t n = (int64_t)vb.b * blockDim.x + threadIdx.x; n < L.nn; n += (int64_t)vb.n * blockDim.x) {
-        const int X = (int)(n % nnx), Y = (int)((n / nnx) % nny), Z = (int)(n / ((int64_t)nnx * nny));
-        float acc0 = 0.0f, acc1 = 0.0f, acc2 = 0.0f;
-#pragma unroll
-        for (int dz = 0; dz <= 1; ++dz)
-#pragma unroll
-            for (int dy = 0; dy <= 1; ++dy)
-#pragma unroll
-                for (int dx = 0; dx <= 1; ++dx) {
-                    const int ex = X - dx, ey = Y - dy, ez = Z - dz;
-                    if (ex < 0 || ey < 0 || ez < 0 || ex >= L.nx || ey >= L.ny || ez >= L.nz) continue;
-                    const int a = corner_of(dx, dy, dz);
-                    const float* K = Kel + ((int64_t)(ez * L.ny + ey) * L.nx + ex);
-#pragma unroll
-                    for (int b = 0; b < 8; ++b) {
-                        const int64_t m = ((int64_t)(ez + corner_dz(b)) * nny + ey + corner_dy(b)) * nnx + ex + corner_dx(b);
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) {
-                            const float xv = x[c * L.cs + m];
-                            acc0 = fmaf(K[sym_pack(3 * a, 3 * b + c) * ne], xv, acc0);
-                            acc1 = fmaf(K[sym_pack(3 * a + 1, 3 * b + c) * ne], xv, acc1);
-                            acc2 = fmaf(K[sym_pack(3 * a + 2, 3 * b + c) * ne], xv, acc2);
-                        }
-                    }
-                }
-        const int mk = L.mask[n];
-        y[n] = (mk & 1) ? 0.0f : acc0;
-        y[L.cs + n] = (mk & 2) ? 0.0f : acc1;
-        y[2 * L.cs + n] = (mk & 4) ? 0.0f : acc2;
+// y = r - K_l x or y = x + w (r - K_l x) / D (y other than x) from the FP32 element matrices of a coarse level,
+// stored symmetric-packed and entry-major (entry p of element e at p * ne + e; the Galerkin operators P^T K P are
+// symmetric).  Fixed DOFs 0.
+struct SymPositions {   // the packed positions of the 24 x 24 entries, in shared memory
+    __align__(16) int pos[24][24];
+    __device__ void fill() {
+        for (int k = threadIdx.x; k < 576; k += blockDim.x) pos[k / 24][k % 24] = sym_pack(k / 24, k % 24);
+        __syncthreads();
     }
+    template <class F>
+    __device__ __forceinline__ void row(int i, int ne, F&& take) const {
+#pragma unroll
+        for (int j = 0; j < 24; j += 4) {
+            const int4 p = *reinterpret_cast<const int4*>(&pos[i][j]);
+            take(j, (int64_t)p.x * ne);
+            take(j + 1, (int64_t)p.y * ne);
+            take(j + 2, (int64_t)p.z * ne);
+            take(j + 3, (int64_t)p.w * ne);
+        }
+    }
+};
+template <LevelOp OP>
+__device__ __forceinline__ void level_store32(const MgLevel32& L, int n, int row, float kx, const float* __restrict__ x,
+                                              const float* __restrict__ r, float* __restrict__ y, float w) {
+    const bool fixed = (L.mask[n] >> row) & 1;
+    const int64_t i = row * L.cs + n;
+    if (OP == LevelOp::Residual) y[i] = fixed ? 0.0f : r[i] - kx;
+    else y[i] = fixed ? 0.0f : x[i] + (w * (r[i] - kx)) * L.diag[i];
 }
-__global__ void k_level_matvec32(MgLevel32 L, const float* __restrict__ Kel, const float* __restrict__ x,
-                                 float* __restrict__ y, const PcgScalars* S) {
-    level_matvec32(vb_real(), L, Kel, x, y, S);
+template <LevelOp OP>
+__device__ __forceinline__ void level_split32(VB vb, const MgLevel32& L, const float* __restrict__ Kel,
+                                              const float* __restrict__ x, const float* __restrict__ r,
+                                              float* __restrict__ y, float w, const PcgScalars* S,
+                                              const SymPositions& sp, float* sums) {
+    if (S->done) return;
+    const int ne = L.nx * L.ny * L.nz;
+    for (int64_t n0 = (int64_t)vb.b * LS_NODES; n0 < L.nn; n0 += (int64_t)vb.n * LS_NODES)
+        level_split<float>(
+            L, L.cs, n0, Kel, x, sums, [&](int i, auto&& take) { sp.row(i, ne, take); },
+            [&](int n, int row, float kx) { level_store32<OP>(L, n, row, kx, x, r, y, w); });
 }
+template <LevelOp OP>
+__global__ void __launch_bounds__(LS_THREADS, 1) k_level_split32(MgLevel32 L, const float* __restrict__ Kel,
+                                                                 const float* __restrict__ x,
+                                                                 const float* __restrict__ r, float* __restrict__ y,
+                                                                 float w, const PcgScalars* S) {
+    __shared__ SymPositions sp;
+    __shared__ float sums[3 * LS_NODES];
+    sp.fill();
+    level_split32<OP>(vb_real(), L, Kel, x, r, y, w, S, sp, sums);
+}
+template <LevelOp OP>
+__global__ void __launch_bounds__(LN_NODES, 3) k_level_nodes32(MgLevel32 L, const float* __restrict__ Kel,
+                                                                 const float* __restrict__ x,
+                                                                 const float* __restrict__ r, float* __restrict__ y,
+                                                                 float w, const PcgScalars* S) {
+    __shared__ SymPositions sp;
+    if (S->done) return;
+    sp.fill();
+    const int ne = L.nx * L.ny * L.nz;
+    const int64_t n = (int64_t)blockIdx.x * LN_NODES + threadIdx.x;
+    if (n >= L.nn) return;
+    float kx[3];
+    level_nodes<3, float>(L, L.cs, (int)n, 0, Kel, x, [&](int i, auto&& take) { sp.row(i, ne, take); }, kx);
+#pragma unroll
+    for (int row = 0; row < 3; ++row) level_store32<OP>(L, (int)n, row, kx[row], x, r, y, w);
+}
+// nodes up to which the split form is used: four waves of its blocks (one per SM).  Measured at 9,537 nodes in FP32:
+// a V-cycle at 256x512x256 2.45 ms split, 2.48 not; at 30,625: 35 us split, 22 not (FP64: 0.764 against 0.731 ms a cycle).
+constexpr int64_t LEVEL_SPLIT_MAX32 = 4 * 148 * LS_NODES;
 
 // FP32 symmetric-packed, entry-major image of element-major FP64 element matrices (the upper triangle):
 // dst[p * ne + e] = src[e * 576 + 24 i + j], (i, j) the p-th upper-triangle entry
@@ -347,13 +373,11 @@ inline unsigned blocks_of(int64_t n, int t) {
 }
 
 // ---------------------------------------------------------------- batched launches (persistent grids)
-__global__ void __launch_bounds__(256) k_batch_level_op32(const BatchLevelOp* __restrict__ a,
-                                                          const int* __restrict__ act, int N, int op) {
-    batch_walk(a, act, N, [&](const BatchLevelOp& A, VB vb) {
+__global__ void __launch_bounds__(256) k_batch_jacobi32(const BatchJacobi* __restrict__ a, const int* __restrict__ act,
+                                                        int N) {
+    batch_walk(a, act, N, [&](const BatchJacobi& A, VB vb) {
         const MgLevel32 L = A.L;
-        if (op == 0) jacobi_init32(vb, L, A.r, A.x, A.w, A.S);
-        else if (op == 1) residual32(vb, L, A.r, A.kx, A.S);
-        else jacobi_correct32(vb, L, A.r, A.kx, A.x, A.w, A.S);
+        jacobi_init32(vb, L, A.r, A.x, A.w, A.S);
     });
 }
 __global__ void __launch_bounds__(256) k_batch_prolong_add32(const BatchProlongAdd* __restrict__ a,
@@ -363,28 +387,33 @@ __global__ void __launch_bounds__(256) k_batch_prolong_add32(const BatchProlongA
         prolong_add32(vb, Lc, Lf, A.xc, A.xi, A.xo, A.S);
     });
 }
-__global__ void __launch_bounds__(128) k_batch_level_matvec32(const BatchLevelMatvec* __restrict__ a,
-                                                              const int* __restrict__ act, int N) {
-    batch_walk(a, act, N, [&](const BatchLevelMatvec& A, VB vb) {
+template <LevelOp OP>
+__global__ void __launch_bounds__(LS_THREADS, 1) k_batch_level_op32(const BatchLevelOp* __restrict__ a,
+                                                                    const int* __restrict__ act, int N) {
+    __shared__ SymPositions sp;
+    __shared__ float sums[3 * LS_NODES];
+    sp.fill();
+    batch_walk(a, act, N, [&](const BatchLevelOp& A, VB vb) {
         const MgLevel32 L = A.L;
-        level_matvec32(vb, L, A.Kel, A.x, A.y, A.S);
+        level_split32<OP>(vb, L, A.Kel, A.x, A.r, A.y, A.w, A.S, sp, sums);
     });
 }
-constexpr int BATCH_GRID256 = 8 * 148, BATCH_GRID128 = 16 * 148;
+constexpr int BATCH_GRID256 = 8 * 148, BATCH_GRID_LS = 148;
 
 }  // namespace
 
-int batch_blocks_level_op(const BatchLevelOp& a) { return (int)blocks_of(a.L.nn, 256); }
+int batch_blocks_jacobi(const BatchJacobi& a) { return (int)blocks_of(a.L.nn, 256); }
 int batch_blocks_prolong_add(const BatchProlongAdd& a) { return (int)blocks_of(a.Lf.nn, 256); }
-int batch_blocks_level_matvec(const BatchLevelMatvec& a) { return (int)blocks_of(a.L.nn, 128); }
-void launch_batch_level_op32(const BatchLevelOp* a, const int* act, int N, int op, cudaStream_t s) {
-    k_batch_level_op32<<<BATCH_GRID256, 256, 0, s>>>(a, act, N, op);
+int batch_blocks_level_op(const BatchLevelOp& a) { return (int)blocks_of(a.L.nn, LS_NODES); }
+void launch_batch_jacobi32(const BatchJacobi* a, const int* act, int N, cudaStream_t s) {
+    k_batch_jacobi32<<<BATCH_GRID256, 256, 0, s>>>(a, act, N);
 }
 void launch_batch_prolong_add32(const BatchProlongAdd* a, const int* act, int N, cudaStream_t s) {
     k_batch_prolong_add32<<<BATCH_GRID256, 256, 0, s>>>(a, act, N);
 }
-void launch_batch_level_matvec32(const BatchLevelMatvec* a, const int* act, int N, cudaStream_t s) {
-    k_batch_level_matvec32<<<BATCH_GRID128, 128, 0, s>>>(a, act, N);
+void launch_batch_level_op32(const BatchLevelOp* a, const int* act, int N, bool correct, cudaStream_t s) {
+    if (correct) k_batch_level_op32<LevelOp::Correct><<<BATCH_GRID_LS, LS_THREADS, 0, s>>>(a, act, N);
+    else k_batch_level_op32<LevelOp::Residual><<<BATCH_GRID_LS, LS_THREADS, 0, s>>>(a, act, N);
 }
 
 void launch_jacobi_init32(const MgLevel32& L, const float* r, float* x, float w, const PcgScalars* S, cudaStream_t s) {
@@ -401,9 +430,17 @@ void launch_prolong_add32(const MgLevel32& Lc, const MgLevel32& Lf, const float*
                           const PcgScalars* S, cudaStream_t s) {
     k_prolong_add32<<<blocks_of(Lf.nn, 256), 256, 0, s>>>(Lc, Lf, xc, xi, xo, S);
 }
-void launch_level_matvec32(const MgLevel32& L, const float* Kel, const float* x, float* y, const PcgScalars* S,
-                           cudaStream_t s) {
-    k_level_matvec32<<<blocks_of(L.nn, 128), 128, 0, s>>>(L, Kel, x, y, S);
+void launch_level_op32(const MgLevel32& L, const float* Kel, const float* x, const float* r, float* y, bool correct,
+                       float w, const PcgScalars* S, cudaStream_t s) {
+    if (L.nn <= LEVEL_SPLIT_MAX32) {
+        const unsigned b = blocks_of(L.nn, LS_NODES);
+        if (correct) k_level_split32<LevelOp::Correct><<<b, LS_THREADS, 0, s>>>(L, Kel, x, r, y, w, S);
+        else k_level_split32<LevelOp::Residual><<<b, LS_THREADS, 0, s>>>(L, Kel, x, r, y, w, S);
+        return;
+    }
+    const unsigned b = (unsigned)((L.nn + LN_NODES - 1) / LN_NODES);
+    if (correct) k_level_nodes32<LevelOp::Correct><<<b, LN_NODES, 0, s>>>(L, Kel, x, r, y, w, S);
+    else k_level_nodes32<LevelOp::Residual><<<b, LN_NODES, 0, s>>>(L, Kel, x, r, y, w, S);
 }
 void launch_kel_pack32(int64_t ne, const double* Kel, float* KelP32, cudaStream_t s) {
     k_kel_pack32<<<(unsigned)((ne + 31) / 32), dim3(32, 8), 0, s>>>(ne, Kel, KelP32);

@@ -203,12 +203,25 @@ __device__ __forceinline__ float hat_sum(int c, int n) {
     return sw;
 }
 
+// a coarse node's restricted residual, masked, and with x0 the Standard cycle's Jacobi start x0 = w0 rc / D
+__device__ __forceinline__ void restrict_store32(const MgLevel32& Lc, int n, float v0, float v1, float v2,
+                                                 float* __restrict__ rc, float* __restrict__ x0, float w0) {
+    const int m = Lc.mask[n];
+    const float v[3] = {(m & 1) ? 0.0f : v0, (m & 2) ? 0.0f : v1, (m & 4) ? 0.0f : v2};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const int64_t i = c * Lc.nn + n;
+        rc[i] = v[c];
+        if (x0) x0[i] = ((m >> c) & 1) ? 0.0f : (w0 * v[c]) * Lc.diag[i];
+    }
+}
+
 // y and z window sums of the x-pass result a1[fz][fy][cx] in one pass, normalised by the summed in-range
 // weights and masked (the k_restrict_y32 + k_restrict_z32 pair fused; one thread per coarse node).
 template <int SP>
 __device__ __forceinline__ void restrict_yz32(VB vb, const MgLevel32& Lc, const MgLevel32& Lf,
                                               const float* __restrict__ a1, float* __restrict__ rc,
-                                              const PcgScalars* S, int normalize) {
+                                              const PcgScalars* S, int normalize, float* __restrict__ x0, float w0) {
     if (S->done) return;
     constexpr int WS = 2 * SP - 1;
     const int n = vb.b * blockDim.x + threadIdx.x;
@@ -240,22 +253,20 @@ __device__ __forceinline__ void restrict_yz32(VB vb, const MgLevel32& Lc, const 
     }
     // normalised average (transfers.cpp:520-528) or, for the Standard cycle, the transposed prolongation
     const float iw = normalize ? 1.0f / (hat_sum<SP>(cz, fnz) * hat_sum<SP>(cy, fny) * hat_sum<SP>(cx, fnx)) : 1.0f;
-    const int m = Lc.mask[n];
-    rc[n] = (m & 1) ? 0.0f : v0 * iw;
-    rc[Lc.nn + n] = (m & 2) ? 0.0f : v1 * iw;
-    rc[2 * Lc.nn + n] = (m & 4) ? 0.0f : v2 * iw;
+    restrict_store32(Lc, n, v0 * iw, v1 * iw, v2 * iw, rc, x0, w0);
 }
 template <int SP>
 __global__ void __launch_bounds__(256) k_restrict_yz32(MgLevel32 Lc, MgLevel32 Lf, const float* __restrict__ a1,
-                                                       float* __restrict__ rc, const PcgScalars* S, int normalize) {
-    restrict_yz32<SP>(vb_real(), Lc, Lf, a1, rc, S, normalize);
+                                                       float* __restrict__ rc, const PcgScalars* S, int normalize,
+                                                       float* __restrict__ x0, float w0) {
+    restrict_yz32<SP>(vb_real(), Lc, Lf, a1, rc, S, normalize, x0, w0);
 }
 
 // The whole 3D window of the fine residual in one pass (levels small enough to sit in L2).
 template <int SP>
 __device__ __forceinline__ void restrict_xyz32(VB vb, const MgLevel32& Lc, const MgLevel32& Lf,
                                                const float* __restrict__ rf, float* __restrict__ rc,
-                                               const PcgScalars* S, int normalize) {
+                                               const PcgScalars* S, int normalize, float* __restrict__ x0, float w0) {
     if (S->done) return;
     constexpr int WS = 2 * SP - 1;
     const int n = vb.b * blockDim.x + threadIdx.x;
@@ -297,15 +308,13 @@ __device__ __forceinline__ void restrict_xyz32(VB vb, const MgLevel32& Lc, const
     }
     // normalised average (transfers.cpp:520-528) or, for the Standard cycle, the transposed prolongation
     const float iw = normalize ? 1.0f / (hat_sum<SP>(cz, fnz) * hat_sum<SP>(cy, fny) * hat_sum<SP>(cx, fnx)) : 1.0f;
-    const int m = Lc.mask[n];
-    rc[n] = (m & 1) ? 0.0f : v0 * iw;
-    rc[Lc.nn + n] = (m & 2) ? 0.0f : v1 * iw;
-    rc[2 * Lc.nn + n] = (m & 4) ? 0.0f : v2 * iw;
+    restrict_store32(Lc, n, v0 * iw, v1 * iw, v2 * iw, rc, x0, w0);
 }
 template <int SP>
 __global__ void __launch_bounds__(256) k_restrict_xyz32(MgLevel32 Lc, MgLevel32 Lf, const float* __restrict__ rf,
-                                                        float* __restrict__ rc, const PcgScalars* S, int normalize) {
-    restrict_xyz32<SP>(vb_real(), Lc, Lf, rf, rc, S, normalize);
+                                                        float* __restrict__ rc, const PcgScalars* S, int normalize,
+                                                        float* __restrict__ x0, float w0) {
+    restrict_xyz32<SP>(vb_real(), Lc, Lf, rf, rc, S, normalize, x0, w0);
 }
 
 // Trilinear prolongation at fine node (fx,fy,fz) from the coarse cell fx >> sh (span 1 << sh), clamped to the
@@ -617,9 +626,9 @@ __global__ void __launch_bounds__(256) k_batch_restrict32(const BatchRestrict* _
         const MgLevel32 Lc = A.Lc, Lf = A.Lf;
         if (Lc.span == 4) {
             if (stage == 0) restrict_x32(vb, Lc, Lf, A.rf, A.a1, A.S);
-            else restrict_yz32<4>(vb, Lc, Lf, A.a1, A.rc, A.S, A.normalize);
+            else restrict_yz32<4>(vb, Lc, Lf, A.a1, A.rc, A.S, A.normalize, A.x0, A.w);
         } else {
-            restrict_xyz32<2>(vb, Lc, Lf, A.rf, A.rc, A.S, A.normalize);
+            restrict_xyz32<2>(vb, Lc, Lf, A.rf, A.rc, A.S, A.normalize, A.x0, A.w);
         }
     });
 }
@@ -728,13 +737,13 @@ void launch_matvec32(const Grid& g, const float* Ke, const float* E, const uint8
 // x pass then a fused y-z pass on the finest transition (span 4); one fused x-y-z pass on the
 // coarser ones (span 2), whose fine residual sits in L2.
 void launch_restrict32(const MgLevel32& Lc, const MgLevel32& Lf, const float* rf, float* rc, float* a1,
-                       const PcgScalars* S, cudaStream_t s, bool normalize) {
+                       const PcgScalars* S, cudaStream_t s, bool normalize, float* x0, float w) {
     const int64_t n1 = (int64_t)(Lf.nz + 1) * (Lf.ny + 1) * (Lc.nx + 1);
     if (Lc.span == 4) {
         k_restrict_x32<<<blocks_for(n1, 256), 256, 0, s>>>(Lc, Lf, rf, a1, S);
-        k_restrict_yz32<4><<<blocks_for(Lc.nn, 256), 256, 0, s>>>(Lc, Lf, a1, rc, S, normalize ? 1 : 0);
+        k_restrict_yz32<4><<<blocks_for(Lc.nn, 256), 256, 0, s>>>(Lc, Lf, a1, rc, S, normalize ? 1 : 0, x0, w);
     } else {
-        k_restrict_xyz32<2><<<blocks_for(Lc.nn, 256), 256, 0, s>>>(Lc, Lf, rf, rc, S, normalize ? 1 : 0);
+        k_restrict_xyz32<2><<<blocks_for(Lc.nn, 256), 256, 0, s>>>(Lc, Lf, rf, rc, S, normalize ? 1 : 0, x0, w);
     }
 }
 void launch_rows_to32(int64_t rows, int len, const double* a, float* b, cudaStream_t s) {

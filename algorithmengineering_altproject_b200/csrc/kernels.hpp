@@ -110,7 +110,8 @@ void launch_diag_coarsen(const MgLevel& Lc, const MgLevel& Lf, cudaStream_t s);
 // separable restriction; a1, a2: pass buffers of 3*(fnz*fny*cnx) and 3*(fnz*cny*cnx) doubles
 // normalize = false: the transpose of the trilinear prolongation (no division by the weight sum)
 void launch_restrict(const MgLevel& Lc, const MgLevel& Lf, const double* rf, double* rc, double* a1, double* a2,
-                     const PcgScalars* S, cudaStream_t s, bool normalize = true);
+                     const PcgScalars* S, cudaStream_t s, bool normalize = true,
+                     double* x0 = nullptr, double w = 0.0);
 void launch_coarse_jacobi(const MgLevel& L, const PcgScalars* S, cudaStream_t s);
 void launch_prolong_smooth(const MgLevel& Lc, const MgLevel& Lf, const double* xc, const double* rf, double* xf,
                            double weight, const PcgScalars* S, cudaStream_t s);
@@ -145,8 +146,9 @@ void launch_galerkin_fine(const Grid& g, const MgLevel& L1, const double* E, con
 void launch_galerkin_coarse(const MgLevel& Lf, const MgLevel& Lc, const double* Kf, double* Kc, cudaStream_t s);
 void launch_level_diag(const MgLevel& L, const double* Kel, cudaStream_t s);
 // KelT: the level's entry-major element matrices
-void launch_level_matvec(const MgLevel& L, const double* KelT, const double* x, double* y, const PcgScalars* S,
-                         cudaStream_t s);
+// y = r - K_l x, or (correct) y = x + w (r - K_l x) / D, from the entry-major element matrices; y must not be x
+void launch_level_op(const MgLevel& L, const double* KelT, const double* x, const double* r, double* y, bool correct,
+                     double w, const PcgScalars* S, cudaStream_t s);
 void launch_jacobi_init(const MgLevel& L, const double* r, double* x, double w, const PcgScalars* S, cudaStream_t s);
 void launch_residual(const MgLevel& L, const double* r, double* kx, const PcgScalars* S, cudaStream_t s);
 void launch_jacobi_correct(const MgLevel& L, const double* r, const double* kx, double* x, double w,
@@ -242,9 +244,9 @@ void launch_mixed_accumulate(const Grid& g, double* u, const float* d, cudaStrea
 void launch_matvec32(const Grid& g, const float* Ke, const float* E, const uint8_t* mask, const float* u, float* y,
                      RedSlot dot, PcgScalars* S, int mark, cudaStream_t s);
 // rc = normalised restriction of rf (normalize = false: the transposed prolongation); a1 holds the x-pass
-// result on span-4 transitions
+// result on span-4 transitions.  With x0, the coarse level's Jacobi start x0 = w rc / D is written too.
 void launch_restrict32(const MgLevel32& Lc, const MgLevel32& Lf, const float* rf, float* rc, float* a1,
-                       const PcgScalars* S, cudaStream_t s, bool normalize = true);
+                       const PcgScalars* S, cudaStream_t s, bool normalize = true, float* x0 = nullptr, float w = 0.0f);
 // FP32 image of `rows` rows of `len` doubles (same layout)
 void launch_rows_to32(int64_t rows, int len, const double* a, float* b, cudaStream_t s);
 // ---- the Standard V-cycle in FP32 (k_mg_standard32.cu)
@@ -255,9 +257,10 @@ void launch_jacobi_correct32(const MgLevel32& L, const float* r, const float* kx
 // xo = xi + P xc (fixed DOFs 0); xo may be xi
 void launch_prolong_add32(const MgLevel32& Lc, const MgLevel32& Lf, const float* xc, const float* xi, float* xo,
                           const PcgScalars* S, cudaStream_t s);
-// KelP32: the level's element matrices as FP32, symmetric-packed (300 upper-triangle entries), entry-major
-void launch_level_matvec32(const MgLevel32& L, const float* KelP32, const float* x, float* y, const PcgScalars* S,
-                           cudaStream_t s);
+// y = r - K_l x, or (correct) y = x + w (r - K_l x) / D; y must not be x.  KelP32: the level's element matrices as
+// FP32, symmetric-packed (300 upper-triangle entries), entry-major
+void launch_level_op32(const MgLevel32& L, const float* KelP32, const float* x, const float* r, float* y, bool correct,
+                       float w, const PcgScalars* S, cudaStream_t s);
 void launch_kel_pack32(int64_t ne, const double* Kel, float* KelP32, cudaStream_t s);
 void launch_dot_rz32(int64_t n3, const float* r, const float* z, RedSlot red, PcgScalars* S, cudaStream_t s);
 void launch_prolong_smooth32(const MgLevel32& Lc, const MgLevel32& Lf, const float* xc, const float* rf, float* xf,
@@ -344,6 +347,8 @@ struct BatchRestrict {    // restriction Lf -> Lc: span 4 x pass rf -> a1 then y
     float* rc;
     PcgScalars* S;
     int normalize;        // 1: the Adapted cycle's weighted average; 0: the Standard cycle's P^T
+    float* x0;            // Standard cycle, above the coarsest level: x0 = w rc / D too
+    float w;
 };
 struct BatchProlong {     // prolongation + smoothing on a level above the finest
     MgLevel32 Lc, Lf;
@@ -365,11 +370,9 @@ struct BatchCoarse {      // coarsest-level solve
     const int* status;
     PcgScalars* S;
 };
-// the Standard V-cycle's level steps (FP32): op 0 x = w r / D, op 1 kx <- r - kx, op 2 x += w (r - kx) / D
-struct BatchLevelOp {
+struct BatchJacobi {      // the Standard cycle's finest-level start x = w r / D
     MgLevel32 L;
     const float* r;
-    float* kx;
     float* x;
     float w;
     PcgScalars* S;
@@ -381,19 +384,21 @@ struct BatchProlongAdd {  // xo = xi + P xc
     float* xo;
     PcgScalars* S;
 };
-struct BatchLevelMatvec { // y = K_l x from the level's FP32 element matrices
+struct BatchLevelOp {     // y = r - K_l x, or y = x + w (r - K_l x) / D, from the level's FP32 element matrices
     MgLevel32 L;
     const float* Kel;
     const float* x;
+    const float* r;
     float* y;
+    float w;
     PcgScalars* S;
 };
-int batch_blocks_level_op(const BatchLevelOp& a);
+int batch_blocks_jacobi(const BatchJacobi& a);
 int batch_blocks_prolong_add(const BatchProlongAdd& a);
-int batch_blocks_level_matvec(const BatchLevelMatvec& a);
-void launch_batch_level_op32(const BatchLevelOp* a, const int* act, int N, int op, cudaStream_t s);
+int batch_blocks_level_op(const BatchLevelOp& a);
+void launch_batch_jacobi32(const BatchJacobi* a, const int* act, int N, cudaStream_t s);
 void launch_batch_prolong_add32(const BatchProlongAdd* a, const int* act, int N, cudaStream_t s);
-void launch_batch_level_matvec32(const BatchLevelMatvec* a, const int* act, int N, cudaStream_t s);
+void launch_batch_level_op32(const BatchLevelOp* a, const int* act, int N, bool correct, cudaStream_t s);
 
 struct BatchCompact {     // one launch list's compaction: act from the done flags of its N instances
     PcgScalars* const* S;   // per position
