@@ -168,10 +168,10 @@ int make_list(Batch* B, const std::vector<T>& a, const std::vector<int>& blocks,
     CHECK(B->dalloc(&L->act, act.size()));
     CHECK(B->dalloc(&db, blocks.size()));
     CHECK(B->dalloc(&dS, S.size()));
-    T3D_CUDA_OK(cudaMemcpy(da, a.data(), a.size() * sizeof(T), cudaMemcpyHostToDevice));
-    T3D_CUDA_OK(cudaMemcpy(L->act, act.data(), act.size() * sizeof(int), cudaMemcpyHostToDevice));
-    T3D_CUDA_OK(cudaMemcpy(db, blocks.data(), blocks.size() * sizeof(int), cudaMemcpyHostToDevice));
-    T3D_CUDA_OK(cudaMemcpy(dS, S.data(), S.size() * sizeof(PcgScalars*), cudaMemcpyHostToDevice));
+    T3D_CUDA_OK(cudaMemcpyAsync(da, a.data(), a.size() * sizeof(T), cudaMemcpyHostToDevice, B->st));
+    T3D_CUDA_OK(cudaMemcpyAsync(L->act, act.data(), act.size() * sizeof(int), cudaMemcpyHostToDevice, B->st));
+    T3D_CUDA_OK(cudaMemcpyAsync(db, blocks.data(), blocks.size() * sizeof(int), cudaMemcpyHostToDevice, B->st));
+    T3D_CUDA_OK(cudaMemcpyAsync(dS, S.data(), S.size() * sizeof(PcgScalars*), cudaMemcpyHostToDevice, B->st));
     L->args = da;
     B->compact.push_back(BatchCompact{dS, db, N, L->act});
     return T3D_OK;
@@ -220,7 +220,7 @@ static int batch_lists(Batch* B) {
         if (!ok) return set_error(T3D_ERR_CUDA, "batch member " + std::to_string(i) + ": tensor maps could not be encoded");
     }
     CHECK(B->dalloc(&B->maps, maps.size()));
-    T3D_CUDA_OK(cudaMemcpy(B->maps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
+    T3D_CUDA_OK(cudaMemcpyAsync(B->maps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice, B->st));
 
     B->maxL = 0;
     B->coarse_max = 0;
@@ -325,14 +325,14 @@ static int batch_lists(Batch* B) {
     std::vector<PcgScalars*> S;
     for (const t3d_context* c : B->m) S.push_back(c->S32);
     CHECK(B->dalloc(&B->dcompact, B->compact.size()));
-    T3D_CUDA_OK(cudaMemcpy(B->dcompact, B->compact.data(), B->compact.size() * sizeof(BatchCompact),
-                           cudaMemcpyHostToDevice));
+    T3D_CUDA_OK(cudaMemcpyAsync(B->dcompact, B->compact.data(), B->compact.size() * sizeof(BatchCompact),
+                                cudaMemcpyHostToDevice, B->st));
     B->iter_kernels += 1;   // the compaction
     CHECK(B->dalloc(&B->dS, S.size()));
-    T3D_CUDA_OK(cudaMemcpy(B->dS, S.data(), S.size() * sizeof(PcgScalars*), cudaMemcpyHostToDevice));
+    T3D_CUDA_OK(cudaMemcpyAsync(B->dS, S.data(), S.size() * sizeof(PcgScalars*), cudaMemcpyHostToDevice, B->st));
     CHECK(B->dalloc(&B->dflags, (size_t)n));
     CHECK(B->dalloc(&B->err, 1));
-    T3D_CUDA_OK(cudaMemset(B->err, 0, sizeof(int)));
+    T3D_CUDA_OK(cudaMemsetAsync(B->err, 0, sizeof(int), B->st));
     T3D_CUDA_OK(cudaMallocHost(&B->hflags, (size_t)n * sizeof(int)));
     T3D_CUDA_OK(cudaMallocHost(&B->hS, (size_t)n * sizeof(PcgScalars)));
     T3D_CUDA_OK(cudaMallocHost(&B->hscal, (size_t)n * sizeof(double)));

@@ -86,7 +86,7 @@ static int upload_gpos(Context* c) {
     const int s1 = c->lv[1].span;
     std::vector<double> G((size_t)s1 * s1 * s1 * 576);
     galerkin_positions(s1, c->Ke_h, G.data());
-    T3D_CUDA_OK(cudaMemcpy(c->Gpos, G.data(), G.size() * sizeof(double), cudaMemcpyHostToDevice));
+    T3D_CUDA_OK(cudaMemcpyAsync(c->Gpos, G.data(), G.size() * sizeof(double), cudaMemcpyHostToDevice, c->st));
     return T3D_OK;
 }
 
@@ -419,7 +419,7 @@ int create(int nely, int nelx, int nelz, const t3d_params* prm, const t3d_proble
         CHECK(c->alloc(&c->ce_acc, g.NE));
         CHECK(c->alloc(&c->one, 1));
         const double one = 1.0;
-        T3D_CUDA_OK(cudaMemcpy(c->one, &one, sizeof one, cudaMemcpyHostToDevice));
+        T3D_CUDA_OK(cudaMemcpyAsync(c->one, &one, sizeof one, cudaMemcpyHostToDevice, c->st));
         T3D_CUDA_OK(cudaMemsetAsync(c->b_cases, 0, (size_t)c->ncases * 3 * g.NN * sizeof(double), c->st));
         T3D_CUDA_OK(cudaMemsetAsync(c->u_cases, 0, (size_t)c->ncases * 3 * g.NN * sizeof(double), c->st));
     }
@@ -477,6 +477,8 @@ int create(int nely, int nelx, int nelz, const t3d_params* prm, const t3d_proble
 }
 
 // ------------------------------------------------------------------ lazily built layout maps
+// Uploads go through the context's own stream, like everything that reads them: a plain cudaMemcpy from pageable
+// memory returns once the host buffer is staged, and the context's stream (non-blocking) would not wait for the rest.
 // Morton order of the solid elements (fea.cpp:289-317): octree walk visiting children in key order
 // (x bit most significant, then y, then z), emitting grid cell indices.
 static void morton_walk(const Context* c, int x0, int y0, int z0, int h, std::vector<int32_t>& out) {
@@ -500,7 +502,8 @@ int ensure_morton(Context* c) {
     c->morton_h.reserve(c->ne);
     morton_walk(c, 0, 0, 0, h, c->morton_h);
     CHECK(c->alloc(&c->morton, c->ne));
-    T3D_CUDA_OK(cudaMemcpy(c->morton, c->morton_h.data(), c->ne * sizeof(int32_t), cudaMemcpyHostToDevice));
+    T3D_CUDA_OK(cudaMemcpyAsync(c->morton, c->morton_h.data(), c->ne * sizeof(int32_t), cudaMemcpyHostToDevice,
+                                c->st));
     return T3D_OK;
 }
 
@@ -513,7 +516,8 @@ static int ensure_free(Context* c) {
         for (int k = 0; k < 3; ++k)
             if (!((m[n] >> k) & 1)) c->free_h.push_back((int32_t)(3 * n + k));
     CHECK(c->alloc(&c->free_d, c->free_h.size()));
-    T3D_CUDA_OK(cudaMemcpy(c->free_d, c->free_h.data(), c->free_h.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+    T3D_CUDA_OK(cudaMemcpyAsync(c->free_d, c->free_h.data(), c->free_h.size() * sizeof(int32_t),
+                                cudaMemcpyHostToDevice, c->st));
     return T3D_OK;
 }
 
@@ -1285,7 +1289,7 @@ int t3d_set_ke(t3d_context* ctx, const double* ke) {
     API_GUARD(ctx);
     if (!ke) return t3d::set_error(T3D_ERR_INVALID, "null Ke");
     std::memcpy(ctx->Ke_h, ke, sizeof ctx->Ke_h);
-    T3D_CUDA_OK(cudaMemcpy(ctx->Ke, ctx->Ke_h, sizeof ctx->Ke_h, cudaMemcpyHostToDevice));
+    T3D_CUDA_OK(cudaMemcpyAsync(ctx->Ke, ctx->Ke_h, sizeof ctx->Ke_h, cudaMemcpyHostToDevice, ctx->st));
     CHECK(t3d::update_ke_pattern(ctx));
     if (ctx->standard) CHECK(t3d::upload_gpos(ctx));   // the Standard V-cycle's level-1 Galerkin products
     ctx->mg_ready = false;   // the hierarchy was built with the old Ke: rebuilt by the next design step or t3d_mg_setup
@@ -1293,7 +1297,7 @@ int t3d_set_ke(t3d_context* ctx, const double* ke) {
     if (ctx->Ke32) {
         float k32[576];
         for (int i = 0; i < 576; ++i) k32[i] = (float)ctx->Ke_h[i];
-        T3D_CUDA_OK(cudaMemcpy(ctx->Ke32, k32, sizeof k32, cudaMemcpyHostToDevice));
+        T3D_CUDA_OK(cudaMemcpyAsync(ctx->Ke32, k32, sizeof k32, cudaMemcpyHostToDevice, ctx->st));
         ctx->modal = ctx->prm.matvec32_form == T3D_MATVEC32_AUTO &&
                      t3d::modal_ke_from(ctx->Ke_h, &ctx->kh, &ctx->modal_off);
     }
@@ -1493,8 +1497,9 @@ int t3d_filter_set_state(t3d_context* ctx, const double* last_x, const double* l
     API_GUARD(ctx);
     if (!last_x || !last_rhs) return t3d::set_error(T3D_ERR_INVALID, "null argument");
     const size_t nb = ctx->g.NN * sizeof(double);
-    T3D_CUDA_OK(cudaMemcpy(ctx->flastx, last_x, nb, cudaMemcpyHostToDevice));
-    T3D_CUDA_OK(cudaMemcpy(ctx->flastrhs, last_rhs, nb, cudaMemcpyHostToDevice));
+    T3D_CUDA_OK(cudaMemcpyAsync(ctx->flastx, last_x, nb, cudaMemcpyHostToDevice, ctx->st));
+    T3D_CUDA_OK(cudaMemcpyAsync(ctx->flastrhs, last_rhs, nb, cudaMemcpyHostToDevice, ctx->st));
+    T3D_CUDA_OK(cudaStreamSynchronize(ctx->st));   // the caller's buffers are free again
     return T3D_OK;
 }
 
@@ -1512,7 +1517,7 @@ int t3d_sensitivity(t3d_context* ctx, const float* xphys, const double* ce, doub
     if (!xphys || !ce || !dc) return t3d::set_error(T3D_ERR_INVALID, "null argument");
     CHECK(t3d::upload_cells_f32(ctx, xphys, ctx->x));
     CHECK(t3d::upload_cells_f64(ctx, ce, ctx->ce));
-    T3D_CUDA_OK(cudaMemcpy(ctx->scal + 4, &c_solid, sizeof(double), cudaMemcpyHostToDevice));
+    T3D_CUDA_OK(cudaMemcpyAsync(ctx->scal + 4, &c_solid, sizeof(double), cudaMemcpyHostToDevice, ctx->st));
     t3d::launch_sens(ctx->g, ctx->solid, ctx->x, ctx->ce, ctx->scal + 4, ctx->prm.E0, ctx->prm.Emin, ctx->prm.penal,
                      ctx->dc, ctx->xdc, ctx->st);
     CHECK(t3d::launch_check("sensitivity"));
