@@ -521,18 +521,15 @@ static int ensure_free(Context* c) {
     return T3D_OK;
 }
 
+// the staging buffer: room for every DOF or element, whichever is more (the maps are built by their users)
 static int ensure_stage(Context* c) {
-    CHECK(ensure_free(c));
-    CHECK(ensure_morton(c));
-    const size_t need = std::max(c->free_h.size(), (size_t)c->ne);
-    if (c->stage_n >= need) return T3D_OK;
-    CHECK(c->alloc(&c->stage, need));
-    c->stage_n = need;
-    return T3D_OK;
+    if (c->stage) return T3D_OK;
+    return c->alloc(&c->stage, std::max((size_t)(3 * c->g.NN), (size_t)c->ne));
 }
 
 // host free vector -> device grid vector (fixed DOFs zero)
 static int upload_free(Context* c, const double* h, double* grid) {
+    CHECK(ensure_free(c));
     CHECK(ensure_stage(c));
     const int64_t nf = (int64_t)c->free_h.size();
     T3D_CUDA_OK(cudaMemsetAsync(grid, 0, 3 * c->g.NN * sizeof(double), c->st));
@@ -541,6 +538,7 @@ static int upload_free(Context* c, const double* h, double* grid) {
     return launch_check("scatter_free");
 }
 static int download_free(Context* c, const double* grid, double* h) {
+    CHECK(ensure_free(c));
     CHECK(ensure_stage(c));
     const int64_t nf = (int64_t)c->free_h.size();
     launch_gather_free(nf, c->free_d, grid, c->g.NN, c->stage, c->st);
@@ -549,6 +547,7 @@ static int download_free(Context* c, const double* grid, double* h) {
     return sync(c);
 }
 static int upload_cells_f64(Context* c, const double* h, double* cells) {
+    CHECK(ensure_morton(c));
     CHECK(ensure_stage(c));
     T3D_CUDA_OK(cudaMemsetAsync(cells, 0, c->g.NE * sizeof(double), c->st));
     T3D_CUDA_OK(cudaMemcpyAsync(c->stage, h, c->ne * sizeof(double), cudaMemcpyHostToDevice, c->st));
@@ -556,6 +555,7 @@ static int upload_cells_f64(Context* c, const double* h, double* cells) {
     return launch_check("cells_from_morton");
 }
 static int download_cells_f64(Context* c, const double* cells, double* h) {
+    CHECK(ensure_morton(c));
     CHECK(ensure_stage(c));
     launch_cells_to_morton_f64(c->ne, c->morton, cells, c->stage, c->st);
     CHECK(launch_check("cells_to_morton"));
@@ -563,6 +563,7 @@ static int download_cells_f64(Context* c, const double* cells, double* h) {
     return sync(c);
 }
 static int upload_cells_f32(Context* c, const float* h, float* cells) {
+    CHECK(ensure_morton(c));
     CHECK(ensure_stage(c));
     float* st = reinterpret_cast<float*>(c->stage);
     T3D_CUDA_OK(cudaMemsetAsync(cells, 0, c->g.NE * sizeof(float), c->st));
@@ -571,6 +572,7 @@ static int upload_cells_f32(Context* c, const float* h, float* cells) {
     return launch_check("cells_from_morton");
 }
 static int download_cells_f32(Context* c, const float* cells, float* h) {
+    CHECK(ensure_morton(c));
     CHECK(ensure_stage(c));
     float* st = reinterpret_cast<float*>(c->stage);
     launch_cells_to_morton_f32(c->ne, c->morton, cells, st, c->st);
@@ -1014,11 +1016,6 @@ static int oc_update(Context* c, float V0) {
 }
 
 // ------------------------------------------------------------------ design loop (driver.cpp:60-216)
-static int fill_cells(Context* c, float v) {
-    std::vector<float> h((size_t)c->ne, v);
-    return upload_cells_f32(c, h.data(), c->x);
-}
-
 // Solves every load case on c->E and leaves the element compliance in c->ce and its E-weighted sum in
 // *C.  Several cases (external models): each is solved from its own previous displacement, and
 // ce = sum_k ce_k / K (TOP3D_XL.m:105,125,605-621); c->b and c->u are left holding case 0.
@@ -1055,14 +1052,11 @@ static int solve_all(Context* c, double tol, int maxit, int* iters, double* C) {
 }
 
 int design_init(Context* c, float V0, double* Csolid) {
-    CHECK(ensure_morton(c));
     c->V0 = V0;
     c->loop = 0;
-    CHECK(fill_cells(c, V0));
-    {   // eleMod = E0 for every element for the solid reference solve (driver.cpp:67, 85-103)
-        std::vector<double> e((size_t)c->ne, (double)c->prm.E0);
-        CHECK(upload_cells_f64(c, e.data(), c->E));
-    }
+    // x = V0, eleMod = E0 for every element for the solid reference solve (driver.cpp:67, 85-103)
+    launch_fill_design(c->g, c->solid, V0, (double)c->prm.E0, c->x, c->E, c->st);
+    c->launches += 1;
     T3D_CUDA_OK(cudaMemsetAsync(c->u, 0, 3 * c->g.NN * sizeof(double), c->st));
     if (c->ncases > 1)
         T3D_CUDA_OK(cudaMemsetAsync(c->u_cases, 0, (size_t)c->ncases * 3 * c->g.NN * sizeof(double), c->st));

@@ -102,7 +102,6 @@ struct Context {
     int32_t* free_d = nullptr;
     std::vector<int32_t> free_h;
     double* stage = nullptr;            // staging buffer for host<->device conversions
-    size_t stage_n = 0;
     // pinned host mirror of small device state
     PcgScalars* S_h = nullptr;
     OcState* OC_h = nullptr;

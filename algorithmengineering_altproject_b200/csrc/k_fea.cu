@@ -243,6 +243,17 @@ __device__ __forceinline__ float pow_rounded(float x, float p) {
 
 __device__ __forceinline__ float clamp01(float v) { return v < 0.0f ? 0.0f : (v > 1.0f ? 1.0f : v); }
 
+// The design loop's start.  12 B written per cell: 0.07 ms at 256x512x256, where filling two host arrays, copying
+// them and scattering them took 0.2 s.
+__global__ void k_fill_design(Grid g, const uint8_t* __restrict__ solid, float x0, double e0, float* __restrict__ x,
+                              double* __restrict__ E) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= g.NE) return;
+    const bool in = solid[i] != 0;
+    x[i] = in ? x0 : 0.0f;
+    E[i] = in ? e0 : 0.0;
+}
+
 // SIMP modulus E = fma(rho^p, E0-Emin, Emin) in float (driver.cpp:117-121)
 __global__ void k_simp(Grid g, const uint8_t* __restrict__ solid, const float* __restrict__ x, float E0, float Emin,
                        float penal, double* __restrict__ E) {
@@ -379,6 +390,9 @@ void launch_compliance64(const Grid& g, const double* Ke, const double* E, const
 void launch_objective(const Grid& g, const double* E, const double* ce, const double* Csolid, RedSlot red,
                       double* obj, cudaStream_t s) {
     k_objective<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, E, ce, Csolid, red, obj);
+}
+void launch_fill_design(const Grid& g, const uint8_t* solid, float x0, double e0, float* x, double* E, cudaStream_t s) {
+    k_fill_design<<<blocks_for(g.NE, 256), 256, 0, s>>>(g, solid, x0, e0, x, E);
 }
 void launch_simp(const Grid& g, const uint8_t* solid, const float* x, float E0, float Emin, float penal, double* E,
                  cudaStream_t s) {

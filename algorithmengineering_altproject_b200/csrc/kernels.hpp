@@ -95,6 +95,8 @@ void launch_matvec64_stream(const Grid& g, const Stream64Tiling& t, const double
 void launch_dot_pcg(const Grid& g, const double* p, const double* Ap, RedSlot red, PcgScalars* S, cudaStream_t s);
 void launch_compliance64(const Grid& g, const double* Ke, const double* E, const double* u, double* ce,
                          RedSlot red, double* C, cudaStream_t s);
+// x = x0 and E = e0 on solid cells, 0 elsewhere
+void launch_fill_design(const Grid& g, const uint8_t* solid, float x0, double e0, float* x, double* E, cudaStream_t s);
 void launch_simp(const Grid& g, const uint8_t* solid, const float* x, float E0, float Emin, float penal, double* E,
                  cudaStream_t s);
 void launch_sens(const Grid& g, const uint8_t* solid, const float* x, const double* ce, const double* Csolid,
