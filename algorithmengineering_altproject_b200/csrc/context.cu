@@ -730,7 +730,12 @@ static void pcg_iteration(Context* c) {
     launch_pcg_direction(c->g, c->z, c->p, c->S, c->st);
 }
 
-static constexpr int PCG_CHUNK = 16;
+// Iterations per graph replay.  The host reads a replay's done flag while the next one runs, so a solve that ends
+// leaves up to two replays of launches that return at once (1-2 us each, 17-33 an iteration), and every replay costs
+// a gap of about 10 us.  The FP32 inner solves are short (20-40 iterations, several per solve): 4 a replay, 74 -> 67
+// ms for a design at 96x192x96 (16, 8, 4, 2: 74.2, 68.5, 66.9, 66.9).  The FP64 solves run for hundreds: 16 (800
+// iterations at 30x60x30: 201 ms against 204 with 4).
+static constexpr int PCG_CHUNK = 16, PCG32_CHUNK = 4;
 
 static int ensure_pcg_graph(Context* c) {
     if (!c->use_graph || c->pcg_graph) return T3D_OK;
@@ -873,9 +878,9 @@ static int ensure_pcg32_graph(Context* c) {
     cudaGraph_t graph;
     const int64_t l0 = c->launches;
     T3D_CUDA_OK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
-    for (int k = 0; k < PCG_CHUNK; ++k) pcg32_iteration(c);
+    for (int k = 0; k < PCG32_CHUNK; ++k) pcg32_iteration(c);
     T3D_CUDA_OK(cudaStreamEndCapture(c->st, &graph));
-    c->pcg32_graph_launches = (c->launches - l0) / PCG_CHUNK;   // kernels per iteration in the graph
+    c->pcg32_graph_launches = (c->launches - l0) / PCG32_CHUNK;   // kernels per iteration in the graph
     c->launches = l0;
     cudaError_t e = cudaGraphInstantiate(&c->pcg32_graph, graph, 0);
     cudaGraphDestroy(graph);
@@ -920,10 +925,10 @@ static int mixed_solve(Context* c, double tol, int maxit, int* iters) {
         int queued = 0, chunk = 0;
         bool done = false;
         while (queued < budget && !done) {
-            const int n = std::min(PCG_CHUNK, budget - queued);
-            if (c->use_graph && n == PCG_CHUNK) {
+            const int n = std::min(PCG32_CHUNK, budget - queued);
+            if (c->use_graph && n == PCG32_CHUNK) {
                 T3D_CUDA_OK(cudaGraphLaunch(c->pcg32_graph, c->st));
-                c->launches += (int64_t)PCG_CHUNK * c->pcg32_graph_launches;
+                c->launches += (int64_t)PCG32_CHUNK * c->pcg32_graph_launches;
             } else {
                 for (int k = 0; k < n; ++k) pcg32_iteration(c);
                 CHECK(launch_check("pcg32 iteration"));
