@@ -44,7 +44,8 @@ static_assert(KE_ND <= KE_MAX_DISTINCT, "distinct-magnitude buffer too small");
 
 constexpr int S64_BX = 32;
 constexpr int S64_BY = 8;
-constexpr int S64_SLAB_MIN = 16;   // planes per slab at least (the slab's first element layer is computed twice)
+constexpr int S64_ITEM_LAYERS = 2;   // a work item's overhead in element layers: its first one is computed twice, and
+                                     // nothing overlaps its first loads
 
 // Shared-memory layout of one CTA, in doubles.
 struct S64 {
@@ -250,10 +251,19 @@ int stream64_tiling(const Grid& g, int dev, Stream64Tiling* t) {
     t->tiles_x = (g.nnx + S64::BX - 2) / (S64::BX - 1);
     t->tiles_y = (g.nny + S64::BY - 2) / (S64::BY - 1);
     const int tiles = t->tiles_x * t->tiles_y;
-    // slabs: about 8 waves of the resident CTAs, slabs of at least S64_SLAB_MIN planes
-    int slabs = std::max(1, (8 * resident + tiles - 1) / tiles);
-    slabs = std::min(slabs, std::max(1, g.nnz / S64_SLAB_MIN));
-    t->slab = (g.nnz + slabs - 1) / slabs;
+    // Planes per slab: a layer of a tile costs an SM about the same time whether one or two CTAs are resident (2.5 us,
+    // half of it the FP64 pipe), so the launch takes as long as the SM with the most layers.  The smallest such maximum
+    // wins: one plane per slab on toy grids (33 -> 15 us at 6x12x6), whole waves of long slabs on large ones.
+    long best = 0;
+    for (int slabs = 1; slabs <= g.nnz; ++slabs) {
+        const int slab = (g.nnz + slabs - 1) / slabs;
+        if (slabs != (g.nnz + slab - 1) / slab) continue;   // the same split as a smaller count
+        const long cost = (long)((tiles * (long)slabs + sms - 1) / sms) * (slab + S64_ITEM_LAYERS);
+        if (best == 0 || cost < best) {
+            best = cost;
+            t->slab = slab;
+        }
+    }
     t->slabs = (g.nnz + t->slab - 1) / t->slab;
     t->items = tiles * t->slabs;
     t->grid = std::min(resident, t->items);
