@@ -256,10 +256,10 @@ static int batch_lists(Batch* B) {
     }, mvb));
     CHECK(list(&B->up, all, [](t3d_context* c, int) {
         return BatchUpdate{c->g.NNp, c->r32, c->Ap32, c->slot[1], c->S32};
-    }, [](const BatchUpdate&) { return batch_blocks_update(); }));
+    }, [](const BatchUpdate& a) { return batch_blocks_update(a.NNp); }));
     CHECK(list(&B->dir, all, [](t3d_context* c, int) {
         return BatchDirection{c->g.NNp, c->z32, c->p32, c->d32, c->S32};
-    }, [](const BatchDirection&) { return batch_blocks_update(); }));
+    }, [](const BatchDirection& a) { return batch_blocks_update(a.NNp); }));
     CHECK(list(&B->co, all, [](t3d_context* c, int) {
         return BatchCoarse{c->lv32[c->nlev - 1], c->Xc, c->Nc, c->chol_status, c->S32};
     }, [](const BatchCoarse& a) { return batch_blocks_coarse(a); }));
@@ -320,7 +320,7 @@ static int batch_lists(Batch* B) {
     } else {
         CHECK(list(&B->p0, all, [](t3d_context* c, int) {
             return BatchProlong0{c->lv32[1], c->lv32[0], c->r32, c->z32, c->prm.mg_weight, c->slot[2], c->S32};
-        }, [](const BatchProlong0&) { return batch_blocks_prolong0(); }));
+        }, [](const BatchProlong0& a) { return batch_blocks_prolong0(a); }));
     }
     std::vector<PcgScalars*> S;
     for (const t3d_context* c : B->m) S.push_back(c->S32);

@@ -381,15 +381,15 @@ void launch_setup_load(const Grid& g, int ix_load, int iz_max, double fz, const 
 }
 void launch_matvec64(const Grid& g, const double* Ke, const double* E, const uint8_t* mask, const double* u,
                      double* y, RedSlot dot, PcgScalars* S, cudaStream_t s) {
-    k_matvec64<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, Ke, E, mask, u, y, dot, S);
+    k_matvec64<<<red_blocks(g.NN), RED_THREADS, 0, s>>>(g, Ke, E, mask, u, y, dot, S);
 }
 void launch_compliance64(const Grid& g, const double* Ke, const double* E, const double* u, double* ce,
                          RedSlot red, double* C, cudaStream_t s) {
-    k_compliance64<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, Ke, E, u, ce, red, C);
+    k_compliance64<<<red_blocks((int64_t)g.nx * g.ny * g.nz), RED_THREADS, 0, s>>>(g, Ke, E, u, ce, red, C);
 }
 void launch_objective(const Grid& g, const double* E, const double* ce, const double* Csolid, RedSlot red,
                       double* obj, cudaStream_t s) {
-    k_objective<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, E, ce, Csolid, red, obj);
+    k_objective<<<red_blocks((int64_t)g.nx * g.ny * g.nz), RED_THREADS, 0, s>>>(g, E, ce, Csolid, red, obj);
 }
 void launch_fill_design(const Grid& g, const uint8_t* solid, float x0, double e0, float* x, double* E, cudaStream_t s) {
     k_fill_design<<<blocks_for(g.NE, 256), 256, 0, s>>>(g, solid, x0, e0, x, E);
@@ -407,7 +407,7 @@ void launch_diag0(const Grid& g, const double* Ke, const double* E, const uint8_
     k_diag0<<<blocks_for(g.NN, 256), 256, 0, s>>>(g, Ke, E, mask, diag);
 }
 void launch_dot(const Grid& g, int ncomp, const double* a, const double* b, RedSlot red, double* out, cudaStream_t s) {
-    k_dot<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, ncomp, a, b, red, out);
+    k_dot<<<red_blocks(g.NN), RED_THREADS, 0, s>>>(g, ncomp, a, b, red, out);
 }
 void launch_scatter_free(int64_t nf, const int32_t* free_dofs, const double* vfree, int64_t NN, double* grid,
                          cudaStream_t s) {

@@ -252,29 +252,29 @@ void launch_filter_rhs(const Grid& g, const uint8_t* solid, const float* src, do
 }
 void launch_filter_norms(const Grid& g, const double* rhs, const double* lastrhs, RedSlot r1, RedSlot r2,
                          FilterScalars* F, cudaStream_t s) {
-    k_filter_norms<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, rhs, lastrhs, r1, r2, F);
+    k_filter_norms<<<red_blocks(g.NN), RED_THREADS, 0, s>>>(g, rhs, lastrhs, r1, r2, F);
 }
 void launch_filter_x0(const Grid& g, const double* lastx, double* x, const FilterScalars* F, cudaStream_t s) {
-    k_filter_x0<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, lastx, x, F);
+    k_filter_x0<<<red_blocks(g.NN), RED_THREADS, 0, s>>>(g, lastx, x, F);
 }
 void launch_filter_matvec(const Grid& g, const uint8_t* solid, const double* kf, const double* x, double* y,
                           RedSlot dot, FilterScalars* F, cudaStream_t s) {
-    k_filter_matvec<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, solid, kf, x, y, dot, F);
+    k_filter_matvec<<<red_blocks(g.NN), RED_THREADS, 0, s>>>(g, solid, kf, x, y, dot, F);
 }
 void launch_filter_r0(const Grid& g, const double* rhs, const double* Ax, const double* fdiag, double* r, double* z,
                       double* p, RedSlot r1, RedSlot r2, FilterScalars* F, cudaStream_t s) {
-    k_filter_r0<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, rhs, Ax, fdiag, r, z, p, r1, r2, F);
+    k_filter_r0<<<red_blocks(g.NN), RED_THREADS, 0, s>>>(g, rhs, Ax, fdiag, r, z, p, r1, r2, F);
 }
 void launch_filter_update(const Grid& g, double* x, double* r, const double* p, const double* Ap, RedSlot red,
                           FilterScalars* F, cudaStream_t s) {
-    k_filter_update<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, x, r, p, Ap, red, F);
+    k_filter_update<<<red_blocks(g.NN), RED_THREADS, 0, s>>>(g, x, r, p, Ap, red, F);
 }
 void launch_filter_precond(const Grid& g, const double* r, const double* fdiag, double* z, RedSlot red,
                            FilterScalars* F, cudaStream_t s) {
-    k_filter_precond<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, r, fdiag, z, red, F);
+    k_filter_precond<<<red_blocks(g.NN), RED_THREADS, 0, s>>>(g, r, fdiag, z, red, F);
 }
 void launch_filter_direction(const Grid& g, const double* z, double* p, const FilterScalars* F, cudaStream_t s) {
-    k_filter_direction<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, z, p, F);
+    k_filter_direction<<<red_blocks(g.NN), RED_THREADS, 0, s>>>(g, z, p, F);
 }
 void launch_filter_to_cells(const Grid& g, const uint8_t* solid, const double* x, float* dst, cudaStream_t s) {
     k_filter_to_cells<<<blocks_for((int64_t)g.nx * g.ny * g.nz, 256), 256, 0, s>>>(g, solid, x, dst);

@@ -284,7 +284,7 @@ void launch_matvec64_stream(const Grid& g, const Stream64Tiling& t, const double
 }
 
 void launch_dot_pcg(const Grid& g, const double* p, const double* Ap, RedSlot red, PcgScalars* S, cudaStream_t s) {
-    k_dot_pcg<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, p, Ap, red, S);
+    k_dot_pcg<<<red_blocks(g.NN), RED_THREADS, 0, s>>>(g, p, Ap, red, S);
 }
 
 }  // namespace t3d

@@ -595,7 +595,7 @@ void launch_prolong_smooth(const MgLevel& Lc, const MgLevel& Lf, const double* x
 }
 void launch_prolong_smooth0(const MgLevel& Lc, const MgLevel& Lf, const double* xc, const double* r, double* z,
                             double weight, RedSlot dot, PcgScalars* S, cudaStream_t s) {
-    k_prolong_smooth0<<<RED_BLOCKS, RED_THREADS, 0, s>>>(Lc, Lf, xc, r, z, weight, dot, S);
+    k_prolong_smooth0<<<red_blocks(Lf.nn), RED_THREADS, 0, s>>>(Lc, Lf, xc, r, z, weight, dot, S);
 }
 void launch_coarse_element_matrices(const Grid& g0, const MgLevel& Lc, int span, const uint8_t* mask0, const double* E,
                                     const double* Ke, double emin, double* Kce, cudaStream_t s) {

@@ -484,7 +484,7 @@ void launch_prolong_add(const MgLevel& Lc, const MgLevel& Lf, const double* xc, 
     k_prolong_add<<<blocks_of(Lf.nn, 256), 256, 0, s>>>(Lc, Lf, xc, xf, S);
 }
 void launch_dot_rz(int64_t NN, const double* r, const double* z, RedSlot red, PcgScalars* S, cudaStream_t s) {
-    k_dot_rz<<<RED_BLOCKS, RED_THREADS, 0, s>>>(NN, r, z, red, S);
+    k_dot_rz<<<red_blocks(NN), RED_THREADS, 0, s>>>(NN, r, z, red, S);
 }
 void launch_to_coarse_layout(const MgLevel& L, const double* Kel, double* Kce, cudaStream_t s) {
     k_to_coarse_layout<<<blocks_of((int64_t)L.nx * L.ny * L.nz * 576, 256), 256, 0, s>>>(L, Kel, Kce);

@@ -446,7 +446,7 @@ void launch_kel_pack32(int64_t ne, const double* Kel, float* KelP32, cudaStream_
     k_kel_pack32<<<(unsigned)((ne + 31) / 32), dim3(32, 8), 0, s>>>(ne, Kel, KelP32);
 }
 void launch_dot_rz32(int64_t n3, const float* r, const float* z, RedSlot red, PcgScalars* S, cudaStream_t s) {
-    k_dot_rz32<<<RED_BLOCKS, RED_THREADS, 0, s>>>(n3, r, z, red, S);
+    k_dot_rz32<<<red_blocks(n3 / 4), RED_THREADS, 0, s>>>(n3, r, z, red, S);
 }
 
 }  // namespace t3d

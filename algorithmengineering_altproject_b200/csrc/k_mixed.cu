@@ -670,8 +670,14 @@ constexpr int BATCH_GRID = 8 * 148;
 
 }  // namespace
 
-int batch_blocks_update() { return RED_BLOCKS; }
-int batch_blocks_prolong0() { return RED_BLOCKS; }
+// blocks of the vector steps (4 values a thread) and of the finest prolongation (a warp per 32 runs of a row)
+static int update32_blocks(int64_t NNp) { return red_blocks(3 * NNp / 4); }
+static int prolong0_blocks(const MgLevel32& Lc, const MgLevel32& Lf) {
+    const int64_t chunks = (Lf.nx / Lc.span + 1 + 31) / 32;
+    return red_blocks(32 * chunks * (Lf.ny + 1) * (Lf.nz + 1));
+}
+int batch_blocks_update(int64_t NNp) { return update32_blocks(NNp); }
+int batch_blocks_prolong0(const BatchProlong0& a) { return prolong0_blocks(a.Lc, a.Lf); }
 int batch_blocks_restrict(const BatchRestrict& a, int stage) {
     const MgLevel32& Lc = a.Lc;
     const MgLevel32& Lf = a.Lf;
@@ -721,10 +727,10 @@ void launch_cells_to32(const Grid& g, const double* a, float* b, cudaStream_t s)
 }
 void launch_mixed_residual(const Grid& g, const double* b, const double* Au, float* r32, float* d32, RedSlot red,
                            double* rn2, cudaStream_t s) {
-    k_mixed_residual<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, b, Au, r32, d32, red, rn2);
+    k_mixed_residual<<<red_blocks(3 * g.NNp), RED_THREADS, 0, s>>>(g, b, Au, r32, d32, red, rn2);
 }
 void launch_mixed_accumulate(const Grid& g, double* u, const float* d, cudaStream_t s) {
-    k_mixed_accumulate<<<RED_BLOCKS, 256, 0, s>>>(g, u, d);
+    k_mixed_accumulate<<<red_blocks(3 * g.NN), 256, 0, s>>>(g, u, d);
 }
 void launch_recip_diag32(int64_t rows, int len, int pitch, const double* d, float* rd, cudaStream_t s) {
     k_recip_diag32<<<RED_BLOCKS, 256, 0, s>>>(rows, len, pitch, d, rd);
@@ -732,7 +738,7 @@ void launch_recip_diag32(int64_t rows, int len, int pitch, const double* d, floa
 
 void launch_matvec32(const Grid& g, const float* Ke, const float* E, const uint8_t* mask, const float* u, float* y,
                      RedSlot dot, PcgScalars* S, int mark, cudaStream_t s) {
-    k_matvec32<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, Ke, E, mask, u, y, dot, S, mark);
+    k_matvec32<<<red_blocks(g.NN), RED_THREADS, 0, s>>>(g, Ke, E, mask, u, y, dot, S, mark);
 }
 // x pass then a fused y-z pass on the finest transition (span 4); one fused x-y-z pass on the
 // coarser ones (span 2), whose fine residual sits in L2.
@@ -755,8 +761,9 @@ void launch_prolong_smooth32(const MgLevel32& Lc, const MgLevel32& Lf, const flo
 }
 void launch_prolong_smooth0_32(const MgLevel32& Lc, const MgLevel32& Lf, const float* xc, const float* r, float* z,
                                float w, RedSlot dot, PcgScalars* S, cudaStream_t s) {
-    if (Lc.span == 4) k_prolong_smooth0_32<4><<<RED_BLOCKS, RED_THREADS, 0, s>>>(Lc, Lf, xc, r, z, w, dot, S);
-    else k_prolong_smooth0_32<2><<<RED_BLOCKS, RED_THREADS, 0, s>>>(Lc, Lf, xc, r, z, w, dot, S);
+    const int b = prolong0_blocks(Lc, Lf);
+    if (Lc.span == 4) k_prolong_smooth0_32<4><<<b, RED_THREADS, 0, s>>>(Lc, Lf, xc, r, z, w, dot, S);
+    else k_prolong_smooth0_32<2><<<b, RED_THREADS, 0, s>>>(Lc, Lf, xc, r, z, w, dot, S);
 }
 void launch_coarse_solve32(const MgLevel32& L, const double* X, int N, const int* status, const PcgScalars* S,
                            cudaStream_t s) {
@@ -768,10 +775,10 @@ void launch_pcg_update32(const Grid& g, float* x, float* r, const float* p, cons
                          PcgScalars* S, cudaStream_t s) {
     (void)x;
     (void)p;
-    k_pcg_update32<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, r, Ap, red, S);
+    k_pcg_update32<<<update32_blocks(g.NNp), RED_THREADS, 0, s>>>(g, r, Ap, red, S);
 }
 void launch_pcg_direction32(const Grid& g, const float* z, float* p, float* x, PcgScalars* S, cudaStream_t s) {
-    k_pcg_direction32<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, z, p, x, S);
+    k_pcg_direction32<<<update32_blocks(g.NNp), RED_THREADS, 0, s>>>(g, z, p, x, S);
 }
 
 }  // namespace t3d

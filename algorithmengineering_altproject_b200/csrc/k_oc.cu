@@ -376,7 +376,7 @@ void launch_dc_scale(const Grid& g, const uint8_t* solid, const float* dcf, cons
 void launch_oc_init(OcState* st, cudaStream_t s) { k_oc_init<<<1, 1, 0, s>>>(st); }
 void launch_oc_pass(const Grid& g, const uint8_t* solid, const float* x, const float* dc, OcState* st, float V0,
                     int64_t ne, RedSlot red, cudaStream_t s) {
-    k_oc_pass<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, solid, x, dc, st, V0, ne, red);
+    k_oc_pass<<<red_blocks((int64_t)g.nx * g.ny * g.nz), RED_THREADS, 0, s>>>(g, solid, x, dc, st, V0, ne, red);
 }
 static int64_t oc_vec8_groups(int64_t ne) { return (ne / 8 + V8_RUN - 1) / V8_RUN; }
 int64_t oc_vec8_bytes(int64_t ne) {
@@ -409,7 +409,7 @@ void launch_oc_vec8_pass(int64_t ne, void* scratch, OcState* st, float V0, RedSl
 void launch_oc_finish(const Grid& g, const uint8_t* solid, float* x, const float* dc, OcState* st, int fp64_sum,
                       int64_t ne, RedSlot r1, RedSlot r2, cudaStream_t s) {
     k_oc_reset_change<<<1, 1, 0, s>>>(st);
-    k_oc_finish<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, solid, x, dc, st, fp64_sum, ne, r1, r2);
+    k_oc_finish<<<red_blocks((int64_t)g.nx * g.ny * g.nz), RED_THREADS, 0, s>>>(g, solid, x, dc, st, fp64_sum, ne, r1, r2);
 }
 void launch_oc_vec8_stats(int64_t ne, const int32_t* morton_cells, const float* x, void* scratch, OcState* st,
                           RedSlot red, cudaStream_t s) {

@@ -78,17 +78,17 @@ __global__ void k_pcg_direction(Grid g, const double* __restrict__ z, double* __
 
 void launch_pcg_init(const Grid& g, const double* b, const double* Ax, double* r, RedSlot red, PcgScalars* S,
                      double tol, cudaStream_t s) {
-    k_pcg_init<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, b, Ax, r, red, S, tol);
+    k_pcg_init<<<red_blocks(g.NN), RED_THREADS, 0, s>>>(g, b, Ax, r, red, S, tol);
 }
 void launch_pcg_start(const Grid& g, const double* z, double* p, cudaStream_t s) {
     cudaMemcpyAsync(p, z, 3 * g.NN * sizeof(double), cudaMemcpyDeviceToDevice, s);
 }
 void launch_pcg_update(const Grid& g, double* x, double* r, const double* p, const double* Ap, RedSlot red,
                        PcgScalars* S, cudaStream_t s) {
-    k_pcg_update<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, x, r, p, Ap, red, S);
+    k_pcg_update<<<red_blocks(g.NN), RED_THREADS, 0, s>>>(g, x, r, p, Ap, red, S);
 }
 void launch_pcg_direction(const Grid& g, const double* z, double* p, PcgScalars* S, cudaStream_t s) {
-    k_pcg_direction<<<RED_BLOCKS, RED_THREADS, 0, s>>>(g, z, p, S);
+    k_pcg_direction<<<red_blocks(3 * g.NN), RED_THREADS, 0, s>>>(g, z, p, S);
 }
 
 }  // namespace t3d

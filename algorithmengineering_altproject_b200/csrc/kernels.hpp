@@ -409,10 +409,10 @@ struct BatchCompact {     // one launch list's compaction: act from the done fla
     int* act;
 };
 // logical block counts of one instance's own launches
-int batch_blocks_update();
+int batch_blocks_update(int64_t NNp);
 int batch_blocks_restrict(const BatchRestrict& a, int stage);   // stage 0: x or x-y-z pass, 1: y-z pass (0 if none)
 int batch_blocks_prolong(const BatchProlong& a);
-int batch_blocks_prolong0();
+int batch_blocks_prolong0(const BatchProlong0& a);
 int batch_blocks_coarse(const BatchCoarse& a);
 // the launches (a, act on the device; N instances in the list)
 void launch_batch_flags(PcgScalars* const* S, int n, int* out, cudaStream_t s);   // out[i] = S[i]->done

@@ -28,6 +28,13 @@ namespace t3d {
 // then the same two-level butterfly).  The result depends only on the vector length.
 constexpr int RED_BLOCKS = 1184;   // 8 x 148 SMs
 constexpr int RED_THREADS = 256;
+// Blocks that have work in a canonical reduction over n items.  The blocks left out would add partials of +0 to the
+// same places of the fold, so the result's bits do not change; 1184 arrivals on one counter take 2-3 us, more than a
+// toy grid's whole reduction (update, dot and r.z at 6x12x6: 9, 7 and 10 us, now 4-5).
+inline int red_blocks(int64_t n) {
+    const int64_t b = (n + RED_THREADS - 1) / RED_THREADS;
+    return (int)(b < 1 ? 1 : b < RED_BLOCKS ? b : RED_BLOCKS);
+}
 
 // Reference local corner order (fea.cpp:257-264): corner a of the element in cell (cx,cy,cz) sits at
 // node (cx+CX[a], cy+CY[a], cz+CZ[a]).
