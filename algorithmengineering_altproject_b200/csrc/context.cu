@@ -142,8 +142,8 @@ static int build_levels(Context* c) {
     for (int l = 0; l + 1 < c->nlev; ++l) {
         const MgLevel &Lf = c->lv[l], &Lc = c->lv[l + 1];
         CHECK(c->alloc(&c->ra1[l], (size_t)3 * (Lf.nz + 1) * (Lf.ny + 1) * (Lc.nx + 1)));
-        CHECK(c->alloc(&c->ra2[l], (size_t)3 * (Lf.nz + 1) * (Lc.ny + 1) * (Lc.nx + 1)));
     }
+    T3D_CUDA_OK(mg_kernel_attributes());
     CHECK(c->alloc(&c->chol_status, 1));
     T3D_CUDA_OK(cudaMemsetAsync(c->chol_status, 0, sizeof(int), c->st));
     for (int l = 0; l + 1 < c->nlev; ++l) launch_mask_restrict(c->lv[l + 1], c->lv[l], c->st);
@@ -670,7 +670,14 @@ int matvec64(Context* c, const double* u, double* y, RedSlot dot, PcgScalars* S)
 // kernels of one V-cycle
 static int vcycle_launches(const Context* c) {
     const int L = c->nlev;
-    return c->standard ? 6 * (L - 1) + 5 : 4 * (L - 1) + 1;
+    int n = 0;
+    if (c->standard) {
+        for (int l = 1; l < L; ++l) n += restrict_launches(c->lv[l]);
+        return n + 3 * (L - 2) + 8;
+    }
+    const int tail = adapted_tail_first(c->lv, L, c->Nc), down = std::min(tail, L - 1);
+    for (int l = 1; l <= down; ++l) n += restrict_launches(c->lv[l]);
+    return n + 1 + down;   // the tail or the coarsest solve, and a prolongation per transition
 }
 
 // The 'Standard' cycle (see k_mg_standard.cu); level 0 uses Ap as scratch (free between the PCG update
@@ -687,7 +694,7 @@ static void vcycle_standard(Context* c, const double* r, double* z, PcgScalars* 
     for (int l = 0; l + 1 < L; ++l) {
         const MgLevel &Lf = c->lv[l], &Lc = c->lv[l + 1];
         if (l > 0) launch_level_op(Lf, c->KelT[l], Lf.x, Lf.r, c->vtmp[l], false, w, S, c->st);
-        launch_restrict(Lc, Lf, l == 0 ? c->Ap : c->vtmp[l], Lc.r, c->ra1[l], c->ra2[l], S, c->st, false,
+        launch_restrict(Lc, Lf, l == 0 ? c->Ap : c->vtmp[l], Lc.r, c->ra1[l], S, c->st, false,
                         l + 2 < L ? Lc.x : nullptr, w);
     }
     launch_coarse_solve(c->lv[L - 1], c->Xc, c->Nc, c->chol_status, S, c->st);
@@ -710,13 +717,15 @@ static void vcycle(Context* c, const double* r, double* z, PcgScalars* S, RedSlo
         vcycle_standard(c, r, z, S, dot);
         return;
     }
-    const int L = c->nlev;
-    c->launches += 4 * (L - 1) + 1;
-    for (int l = 0; l + 1 < L; ++l)
-        launch_restrict(c->lv[l + 1], c->lv[l], l == 0 ? r : c->lv[l].r, c->lv[l + 1].r, c->ra1[l], c->ra2[l], S,
-                        c->st);
-    launch_coarse_solve(c->lv[L - 1], c->Xc, c->Nc, c->chol_status, S, c->st);
-    for (int l = L - 2; l >= 1; --l)
+    const int L = c->nlev, tail = adapted_tail_first(c->lv, L, c->Nc), down = std::min(tail, L - 1);
+    c->launches += vcycle_launches(c);
+    for (int l = 0; l < down; ++l)
+        launch_restrict(c->lv[l + 1], c->lv[l], l == 0 ? r : c->lv[l].r, c->lv[l + 1].r, c->ra1[l], S, c->st);
+    if (tail < L)
+        launch_adapted_tail(c->lv, L, tail, c->Xc, c->Nc, c->chol_status, (double)c->prm.mg_weight, S, c->st);
+    else
+        launch_coarse_solve(c->lv[L - 1], c->Xc, c->Nc, c->chol_status, S, c->st);
+    for (int l = down - 1; l >= 1; --l)
         launch_prolong_smooth(c->lv[l + 1], c->lv[l], c->lv[l + 1].x, c->lv[l].r, c->lv[l].x,
                               (double)c->prm.mg_weight, S, c->st);
     launch_prolong_smooth0(c->lv[1], c->lv[0], c->lv[1].x, r, z, (double)c->prm.mg_weight, dot, S, c->st);

@@ -71,8 +71,7 @@ struct Context {
     double* Kd = nullptr;       // [KE_MAX_DISTINCT]
     RedSlot slot[4]{};
     double *Kce = nullptr, *Kc = nullptr, *LT = nullptr, *Lrow = nullptr, *Xc = nullptr;
-    double* ra1[8]{};           // separable-restriction pass buffers per level transition
-    double* ra2[8]{};
+    double* ra1[8]{};           // x-pass buffer of the separable restriction per level transition
     int* chol_status = nullptr;
     double *frhs = nullptr, *fx = nullptr, *fr = nullptr, *fz = nullptr, *fp = nullptr, *fAp = nullptr,
            *flastx = nullptr, *flastrhs = nullptr, *fdiag = nullptr;

@@ -141,141 +141,155 @@ __global__ void k_restrict_x(MgLevel Lc, MgLevel Lf, const double* __restrict__ 
     a1[2 * total + t] = v2;
 }
 
-__global__ void k_restrict_y(MgLevel Lc, MgLevel Lf, const double* __restrict__ a1, double* __restrict__ a2,
-                             const PcgScalars* S) {
-    if (S != nullptr && S->done) return;
-    const int cnx = Lc.nx + 1, cny = Lc.ny + 1, fny = Lf.ny + 1, fnz = Lf.nz + 1;
-    const int64_t total = (int64_t)fnz * cny * cnx, total1 = (int64_t)fnz * fny * cnx;
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= total) return;
-    const int cx = (int)(t % cnx);
-    const int cy = (int)((t / cnx) % cny);
-    const int fz = (int)(t / ((int64_t)cnx * cny));
-    const int s = Lc.span, ws = 2 * s - 1;
-    double v0 = 0.0, v1 = 0.0, v2 = 0.0;
-    for (int iy = 0; iy < ws; ++iy) {
-        const int fy = cy * s + iy - (s - 1);
-        if (fy < 0 || fy >= fny) continue;
-        const double w = hat(iy, s);
-        const int64_t i = ((int64_t)fz * fny + fy) * cnx + cx;
-        v0 = v0 + w * a1[i];
-        v1 = v1 + w * a1[total1 + i];
-        v2 = v2 + w * a1[2 * total1 + i];
+// sum of the in-range hat weights of coarse index c's window over n fine points
+__device__ __forceinline__ double hat_sum(int c, int s, int n) {
+    double sw = 0.0;
+    for (int i = 0; i < 2 * s - 1; ++i) {
+        const int f = c * s + i - (s - 1);
+        if (f >= 0 && f < n) sw = sw + hat(i, s);
     }
-    a2[t] = v0;
-    a2[total + t] = v1;
-    a2[2 * total + t] = v2;
+    return sw;
 }
 
-// normalize = 0: the plain hat-weighted sum, i.e. the transpose of the trilinear prolongation (the
-// 'Standard' V-cycle option)
-__global__ void k_restrict_z(MgLevel Lc, MgLevel Lf, const double* __restrict__ a2, double* __restrict__ rc,
-                             const PcgScalars* S, int normalize, double* __restrict__ x0, double w0) {
+// component c of a coarse node from its window sum: scaled by 1/wSum and masked.  normalize = 0: the plain
+// hat-weighted sum, i.e. the transpose of the trilinear prolongation (the 'Standard' V-cycle option).
+__device__ __forceinline__ double restrict_scale(const MgLevel& Lc, const MgLevel& Lf, int n, int cx, int cy, int cz,
+                                                 int c, double v, int normalize) {
+    const int s = Lc.span;
+    double o = 0.0;
+    if (!normalize) {
+        o = v;
+    } else {
+        const double wsum = hat_sum(cz, s, Lf.nz + 1) * hat_sum(cy, s, Lf.ny + 1) * hat_sum(cx, s, Lf.nx + 1);
+        if (wsum > 1e-12) o = v * (1.0 / wsum);
+    }
+    return ((Lc.mask[n] >> c) & 1) ? 0.0 : o;
+}
+__device__ __forceinline__ void restrict_store(const MgLevel& Lc, int n, int c, double o, double* __restrict__ rc,
+                                               double* __restrict__ x0, double w0) {
+    const int64_t i = c * Lc.nn + n;
+    rc[i] = o;
+    if (x0) {   // the Standard cycle's Jacobi start x0 = w0 rc / D
+        const double d = Lc.diag[i];
+        x0[i] = ((Lc.mask[n] >> c) & 1) ? 0.0 : (w0 * o) * (1.0 / (1.0e-30 < d ? d : 1.0e-30));
+    }
+}
+
+// The y and z sums of a span-SP transition from the x pass, one thread per coarse node and component (blockIdx.y):
+// the y sum of each fine z first, then the z sum, as three separate passes would add them.
+template <int SP>
+__global__ void __launch_bounds__(128) k_restrict_yz(MgLevel Lc, MgLevel Lf, const double* __restrict__ a1,
+                                                     double* __restrict__ rc, const PcgScalars* S, int normalize,
+                                                     double* __restrict__ x0, double w0) {
     if (S != nullptr && S->done) return;
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int WS = 2 * SP - 1;
+    const int n = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
+    if (n >= Lc.nn) return;
+    const int cnx = Lc.nx + 1, cny = Lc.ny + 1, fny = Lf.ny + 1, fnz = Lf.nz + 1;
+    const int cx = n % cnx, cy = (n / cnx) % cny, cz = n / (cnx * cny);
+    const double* __restrict__ a = a1 + c * ((int64_t)fnz * fny * cnx) + cx;
+    double v = 0.0;
+#pragma unroll
+    for (int iz = 0; iz < WS; ++iz) {
+        const int fz = cz * SP + iz - (SP - 1);
+        const bool zin = fz >= 0 && fz < fnz;
+        double q[WS];
+#pragma unroll
+        for (int iy = 0; iy < WS; ++iy) {   // points outside the grid load nothing and add +0, which changes no sum
+            const int fy = cy * SP + iy - (SP - 1);
+            q[iy] = zin && fy >= 0 && fy < fny ? a[(fz * fny + fy) * cnx] : 0.0;
+        }
+        double t = 0.0;
+#pragma unroll
+        for (int iy = 0; iy < WS; ++iy) t = t + hat(iy, SP) * q[iy];
+        v = v + hat(iz, SP) * t;
+    }
+    restrict_store(Lc, n, c, restrict_scale(Lc, Lf, n, cx, cy, cz, c, v, normalize), rc, x0, w0);
+}
+
+// The 27-point window of a span-2 transition in the same nested order, from one component's residual
+__device__ __forceinline__ double window2(const MgLevel& Lc, const MgLevel& Lf, int cx, int cy, int cz,
+                                          const double* rf) {
+    const int fnx = Lf.nx + 1, fny = Lf.ny + 1, fnz = Lf.nz + 1;
+    double q[27];
+#pragma unroll
+    for (int k = 0; k < 27; ++k) {
+        const int fx = cx * 2 + k % 3 - 1, fy = cy * 2 + (k / 3) % 3 - 1, fz = cz * 2 + k / 9 - 1;
+        const bool in = fx >= 0 && fx < fnx && fy >= 0 && fy < fny && fz >= 0 && fz < fnz;
+        q[k] = in ? rf[(fz * fny + fy) * fnx + fx] : 0.0;
+    }
+    double v = 0.0;
+#pragma unroll
+    for (int iz = 0; iz < 3; ++iz) {
+        double t = 0.0;
+#pragma unroll
+        for (int iy = 0; iy < 3; ++iy) {
+            double p = 0.0;
+#pragma unroll
+            for (int ix = 0; ix < 3; ++ix) p = p + hat(ix, 2) * q[9 * iz + 3 * iy + ix];
+            t = t + hat(iy, 2) * p;
+        }
+        v = v + hat(iz, 2) * t;
+    }
+    return v;
+}
+__global__ void __launch_bounds__(128) k_restrict_xyz2(MgLevel Lc, MgLevel Lf, const double* __restrict__ rf,
+                                                       double* __restrict__ rc, const PcgScalars* S, int normalize,
+                                                       double* __restrict__ x0, double w0) {
+    if (S != nullptr && S->done) return;
+    const int n = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
     if (n >= Lc.nn) return;
     const int cnx = Lc.nx + 1, cny = Lc.ny + 1;
-    const int fnx = Lf.nx + 1, fny = Lf.ny + 1, fnz = Lf.nz + 1;
     const int cx = n % cnx, cy = (n / cnx) % cny, cz = n / (cnx * cny);
-    const int s = Lc.span, ws = 2 * s - 1;
-    const int64_t total2 = (int64_t)fnz * cny * cnx;
-    double swx = 0.0, swy = 0.0, swz = 0.0;
-    for (int i = 0; i < ws; ++i) {
-        const int fx = cx * s + i - (s - 1), fy = cy * s + i - (s - 1);
-        if (fx >= 0 && fx < fnx) swx = swx + hat(i, s);
-        if (fy >= 0 && fy < fny) swy = swy + hat(i, s);
-    }
-    double v0 = 0.0, v1 = 0.0, v2 = 0.0;
-    for (int iz = 0; iz < ws; ++iz) {
-        const int fz = cz * s + iz - (s - 1);
-        if (fz < 0 || fz >= fnz) continue;
-        swz = swz + hat(iz, s);
-        const double w = hat(iz, s);
-        const int64_t i = ((int64_t)fz * cny + cy) * cnx + cx;
-        v0 = v0 + w * a2[i];
-        v1 = v1 + w * a2[total2 + i];
-        v2 = v2 + w * a2[2 * total2 + i];
-    }
-    const double wsum = swz * swy * swx;
-    double o0 = 0.0, o1 = 0.0, o2 = 0.0;
-    if (!normalize) {
-        o0 = v0;
-        o1 = v1;
-        o2 = v2;
-    } else if (wsum > 1e-12) {
-        const double iw = 1.0 / wsum;
-        o0 = v0 * iw;
-        o1 = v1 * iw;
-        o2 = v2 * iw;
-    }
-    const int m = Lc.mask[n];
-    const double o[3] = {(m & 1) ? 0.0 : o0, (m & 2) ? 0.0 : o1, (m & 4) ? 0.0 : o2};
-    for (int c = 0; c < 3; ++c) {
-        const int64_t i = c * Lc.nn + n;
-        rc[i] = o[c];
-        if (x0) {   // the Standard cycle's Jacobi start x0 = w0 rc / D
-            const double d = Lc.diag[i];
-            x0[i] = ((m >> c) & 1) ? 0.0 : (w0 * o[c]) * (1.0 / (1.0e-30 < d ? d : 1.0e-30));
-        }
-    }
-}
-
-// coarsest Jacobi fallback x = r/max(1e-30,D) without weight, masked (preconditioner.cpp:199-227)
-__global__ void k_coarse_jacobi(MgLevel L, const PcgScalars* S) {
-    if (S != nullptr && S->done) return;
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= L.nn) return;
-    const int m = L.mask[n];
-    for (int c = 0; c < 3; ++c) {
-        const double d = L.diag[c * L.nn + n];
-        const double dd = 1.0e-30 < d ? d : 1.0e-30;
-        L.x[c * L.nn + n] = ((m >> c) & 1) ? 0.0 : L.r[c * L.nn + n] / dd;
-    }
+    const double v = window2(Lc, Lf, cx, cy, cz, rf + c * Lf.nn);
+    restrict_store(Lc, n, c, restrict_scale(Lc, Lf, n, cx, cy, cz, c, v, normalize), rc, x0, w0);
 }
 
 // trilinear prolongation from the coarse cell floor(f/s), clamped to the last cell
 // (transfers.cpp:378-445), then x = ((w r/D) + P x_c) + (w r/D), 0 on fixed DOFs
 // (preconditioner.cpp:163-173, 230-253).
-__device__ __forceinline__ void prolong_node(const MgLevel& Lc, int s, const double* __restrict__ xc, int fx, int fy,
-                                             int fz, double P[3]) {
-    const int cnx = Lc.nx + 1, cny = Lc.ny + 1;
-    int cx = fx / s, cy = fy / s, cz = fz / s;
-    int rx = fx % s, ry = fy % s, rz = fz % s;
-    if (cx >= Lc.nx) { cx = Lc.nx - 1; rx = s; }
-    if (cy >= Lc.ny) { cy = Lc.ny - 1; ry = s; }
-    if (cz >= Lc.nz) { cz = Lc.nz - 1; rz = s; }
-    const double inv = 1.0 / s;
-    const double wx1 = rx * inv, wx0 = 1.0 - wx1;
-    const double wy1 = ry * inv, wy0 = 1.0 - wy1;
-    const double wz1 = rz * inv, wz0 = 1.0 - wz1;
-    const int b = (cz * cny + cy) * cnx + cx;
-    const int pz = cnx * cny;
-    const int n000 = b, n100 = b + 1, n010 = b + cnx, n110 = b + cnx + 1;
-    for (int c = 0; c < 3; ++c) {
-        const double* X = xc + c * Lc.nn;
-        P[c] = X[n000] * wx0 * wy0 * wz0 + X[n100] * wx1 * wy0 * wz0 + X[n010] * wx0 * wy1 * wz0 +
+struct ProlongAt {   // a fine node's coarse cell and weights
+    int b, py, pz;   // lowest corner, y and z strides
+    double wx0, wx1, wy0, wy1, wz0, wz1;
+    __device__ __forceinline__ ProlongAt(const MgLevel& Lc, int s, int fx, int fy, int fz) {
+        const int cnx = Lc.nx + 1, cny = Lc.ny + 1;
+        int cx = fx / s, cy = fy / s, cz = fz / s;
+        int rx = fx % s, ry = fy % s, rz = fz % s;
+        if (cx >= Lc.nx) { cx = Lc.nx - 1; rx = s; }
+        if (cy >= Lc.ny) { cy = Lc.ny - 1; ry = s; }
+        if (cz >= Lc.nz) { cz = Lc.nz - 1; rz = s; }
+        const double inv = 1.0 / s;
+        wx1 = rx * inv; wx0 = 1.0 - wx1;
+        wy1 = ry * inv; wy0 = 1.0 - wy1;
+        wz1 = rz * inv; wz0 = 1.0 - wz1;
+        b = (cz * cny + cy) * cnx + cx;
+        py = cnx;
+        pz = cnx * cny;
+    }
+    __device__ __forceinline__ double operator()(const double* X) const {
+        const int n000 = b, n100 = b + 1, n010 = b + py, n110 = b + py + 1;
+        return X[n000] * wx0 * wy0 * wz0 + X[n100] * wx1 * wy0 * wz0 + X[n010] * wx0 * wy1 * wz0 +
                X[n110] * wx1 * wy1 * wz0 + X[n000 + pz] * wx0 * wy0 * wz1 + X[n100 + pz] * wx1 * wy0 * wz1 +
                X[n010 + pz] * wx0 * wy1 * wz1 + X[n110 + pz] * wx1 * wy1 * wz1;
     }
+};
+// x = ((w r/D) + P) + (w r/D), 0 on a fixed DOF
+__device__ __forceinline__ double smooth(double w, double r, double d, double P, bool fixed) {
+    const double t = w * r / (1.0e-30 < d ? d : 1.0e-30);
+    return fixed ? 0.0 : (t + P) + t;
 }
 
-__global__ void k_prolong_smooth(MgLevel Lc, MgLevel Lf, const double* __restrict__ xc,
-                                 const double* __restrict__ rf, double* __restrict__ xf, double w,
-                                 const PcgScalars* S) {
+// one thread per node and component (blockIdx.y)
+__global__ void __launch_bounds__(128) k_prolong_smooth(MgLevel Lc, MgLevel Lf, const double* __restrict__ xc,
+                                                        const double* __restrict__ rf, double* __restrict__ xf,
+                                                        double w, const PcgScalars* S) {
     if (S != nullptr && S->done) return;
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+    const int n = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
     if (n >= Lf.nn) return;
     const int fnx = Lf.nx + 1, fny = Lf.ny + 1;
-    const int fx = n % fnx, fy = (n / fnx) % fny, fz = n / (fnx * fny);
-    double P[3];
-    prolong_node(Lc, Lc.span, xc, fx, fy, fz, P);
-    const int m = Lf.mask[n];
-    for (int c = 0; c < 3; ++c) {
-        const double d = Lf.diag[c * Lf.nn + n];
-        const double dd = 1.0e-30 < d ? d : 1.0e-30;
-        const double t = w * rf[c * Lf.nn + n] / dd;
-        xf[c * Lf.nn + n] = ((m >> c) & 1) ? 0.0 : (t + P[c]) + t;
-    }
+    const ProlongAt P(Lc, Lc.span, n % fnx, (n / fnx) % fny, n / (fnx * fny));
+    const int64_t i = c * Lf.nn + n;
+    xf[i] = smooth(w, rf[i], Lf.diag[i], P(xc + c * Lc.nn), (Lf.mask[n] >> c) & 1);
 }
 
 // level 0: writes z and forms r.z in the canonical order; the last block sets rz (first use) or
@@ -289,16 +303,11 @@ __global__ void __launch_bounds__(RED_THREADS) k_prolong_smooth0(MgLevel Lc, MgL
     const int fnx = Lf.nx + 1, fny = Lf.ny + 1;
     double part = 0.0;
     for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < NN; n += gridDim.x * blockDim.x) {
-        const int fx = n % fnx, fy = (n / fnx) % fny, fz = n / (fnx * fny);
-        double P[3];
-        prolong_node(Lc, Lc.span, xc, fx, fy, fz, P);
+        const ProlongAt P(Lc, Lc.span, n % fnx, (n / fnx) % fny, n / (fnx * fny));
         const int m = Lf.mask[n];
         for (int c = 0; c < 3; ++c) {
-            const double d = Lf.diag[c * (int64_t)NN + n];
-            const double dd = 1.0e-30 < d ? d : 1.0e-30;
             const double rv = r[c * (int64_t)NN + n];
-            const double t = w * rv / dd;
-            const double zv = ((m >> c) & 1) ? 0.0 : (t + P[c]) + t;
+            const double zv = smooth(w, rv, Lf.diag[c * (int64_t)NN + n], P(xc + c * Lc.nn), (m >> c) & 1);
             z[c * (int64_t)NN + n] = zv;
             part = part + rv * zv;
         }
@@ -542,30 +551,127 @@ __global__ void __launch_bounds__(INV_WARPS * 32) k_coarse_inverse(const double*
 
 // Coarsest solve x_i = sum_j X[i][j] r_j (sequential in j) when the factorisation succeeded, else
 // the Jacobi fallback x = r/max(1e-30,D) (preconditioner.cpp:195-215); masked (:217-227).
-__global__ void __launch_bounds__(128) k_coarse_solve(MgLevel L, const double* __restrict__ X, int N,
-                                                      const int* __restrict__ status, const PcgScalars* S) {
+// The sum over j is one chain of additions per output, but its products are independent: a block of 32 outputs forms
+// the products of CS_ROWS values of j at a time in shared memory with all its threads (eight loads of a thread in
+// flight instead of one load per addition), then one thread per output adds them in order.
+__device__ __forceinline__ double coarse_jacobi(double r, double d, bool fixed) {
+    return fixed ? 0.0 : r / (1.0e-30 < d ? d : 1.0e-30);
+}
+constexpr int CS_THREADS = 512, CS_ROWS = 128;   // 32 outputs a block: 16 rows at a time, 32 KB of products
+__global__ void __launch_bounds__(CS_THREADS) k_coarse_solve(MgLevel L, const double* __restrict__ X, int N,
+                                                             const int* __restrict__ status, const PcgScalars* S) {
     extern __shared__ double rs[];
     if (S != nullptr && S->done) return;
     const int64_t nn = L.nn;
     if (*status != 1) {
-        for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < nn; n += (int64_t)gridDim.x * blockDim.x) {
-            const int m = L.mask[n];
-            for (int c = 0; c < 3; ++c) {
-                const double d = L.diag[c * nn + n];
-                const double dd = 1.0e-30 < d ? d : 1.0e-30;
-                L.x[c * nn + n] = ((m >> c) & 1) ? 0.0 : L.r[c * nn + n] / dd;
-            }
-        }
+        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < 3 * nn; i += (int64_t)gridDim.x * blockDim.x)
+            L.x[i] = coarse_jacobi(L.r[i], L.diag[i], (L.mask[i % nn] >> (i / nn)) & 1);
         return;
     }
     for (int j = threadIdx.x; j < N; j += blockDim.x) rs[j] = L.r[(j % 3) * nn + j / 3];
     __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
+    double* prod = rs + N;
     double acc = 0.0;
-    for (int j = 0; j < N; ++j) acc = acc + X[(int64_t)j * N + i] * rs[j];
+    for (int j0 = 0; j0 < N; j0 += CS_ROWS) {
+        double q[CS_ROWS / (CS_THREADS / 32)];
+#pragma unroll
+        for (int k = 0; k < CS_ROWS / (CS_THREADS / 32); ++k) {
+            const int j = j0 + k * (CS_THREADS / 32) + warp;
+            q[k] = j < N && i < N ? X[(int64_t)j * N + i] * rs[j] : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < CS_ROWS / (CS_THREADS / 32); ++k) prod[(k * (CS_THREADS / 32) + warp) * 32 + lane] = q[k];
+        __syncthreads();
+        if (warp == 0) {
+            const int nr = min(CS_ROWS, N - j0);
+#pragma unroll 8
+            for (int j = 0; j < nr; ++j) acc = acc + prod[j * 32 + lane];
+        }
+        __syncthreads();
+    }
+    if (warp != 0 || i >= N) return;
     const int ni = i / 3, ci = i % 3;
     L.x[ci * nn + ni] = ((L.mask[ni] >> ci) & 1) ? 0.0 : acc;
+}
+
+// The Adapted cycle below a small level in one block: residuals restricted level by level, the coarsest solve, and
+// prolongation with smoothing back up, all in shared memory, with the separate kernels' operations and order; the
+// coarsest inverse is copied in while the residuals are restricted.  Replaces 2 (T - 1) + 1 launches for T levels.
+// Levels of at most TAIL_NODES nodes and a coarsest system of at most TAIL_N, as long as all of it fits: above that
+// one SM needs longer for the data than the launches take.  With it, two transfer kernels per level fewer and the
+// predicated windows, a V-cycle takes 73 -> 41 us at 30x60x30 and 105 -> 68 us at 64x128x64.
+constexpr int TAIL_NODES = 1536, TAIL_N = 160, TAIL_THREADS = 1024, TAIL_SMEM = 227 * 1024;
+struct TailLevels {
+    MgLevel lv[8];
+    int n;
+};
+__global__ void __launch_bounds__(TAIL_THREADS, 1) k_adapted_tail(TailLevels T, const double* __restrict__ X, int N,
+                                                                  const int* __restrict__ status, double w,
+                                                                  const PcgScalars* S) {
+    extern __shared__ __align__(16) double sm[];
+    if (S != nullptr && S->done) return;
+    double* Xs = sm;                           // the coarsest inverse (N x N, rounded up to whole 16 bytes)
+    double* r = sm + (((int64_t)N * N + 1) & ~1ll);   // level residuals, level solutions; rs in the latter
+    for (int i = threadIdx.x; i < (N * N) / 2; i += TAIL_THREADS)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(Xs + 2 * i)),
+                     "l"(X + 2 * i)
+                     : "memory");
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    if (((N * N) & 1) && threadIdx.x == 0) Xs[N * N - 1] = X[N * N - 1];
+    const MgLevel& L0 = T.lv[0];
+    for (int i = threadIdx.x; i < 3 * (int)L0.nn; i += TAIL_THREADS) r[i] = L0.r[i];
+    __syncthreads();
+    int off = 0;      // of level l's residual
+    for (int l = 0; l + 1 < T.n; ++l) {
+        const MgLevel &Lf = T.lv[l], &Lc = T.lv[l + 1];
+        const int cnx = Lc.nx + 1, cny = Lc.ny + 1, nn = (int)Lc.nn, next = off + 3 * (int)Lf.nn;
+        for (int i = threadIdx.x; i < 3 * nn; i += TAIL_THREADS) {
+            const int c = i / nn, n = i - c * nn;
+            const int cx = n % cnx, cy = (n / cnx) % cny, cz = n / (cnx * cny);
+            const double v = window2(Lc, Lf, cx, cy, cz, r + off + c * Lf.nn);
+            r[next + i] = restrict_scale(Lc, Lf, n, cx, cy, cz, c, v, 1);
+        }
+        __syncthreads();
+        off = next;
+    }
+    const MgLevel& LL = T.lv[T.n - 1];
+    const int nL = (int)LL.nn;
+    double* x = r + off + 3 * nL;   // level l's solution; moves on as the cycle goes up
+    if (*status != 1) {
+        for (int i = threadIdx.x; i < 3 * nL; i += TAIL_THREADS)
+            x[i] = coarse_jacobi(r[off + i], LL.diag[i], (LL.mask[i % nL] >> (i / nL)) & 1);
+    } else {
+        double* rs = x + 3 * nL;
+        for (int j = threadIdx.x; j < N; j += TAIL_THREADS) rs[j] = r[off + (j % 3) * nL + j / 3];
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();
+        const int i = threadIdx.x;
+        if (i < N) {
+            double acc = 0.0;
+#pragma unroll 9
+            for (int j = 0; j < N; ++j) acc = acc + Xs[j * N + i] * rs[j];
+            x[(i % 3) * nL + i / 3] = ((LL.mask[i / 3] >> (i % 3)) & 1) ? 0.0 : acc;
+        }
+    }
+    __syncthreads();
+    for (int l = T.n - 2; l >= 0; --l) {
+        const MgLevel &Lf = T.lv[l], &Lc = T.lv[l + 1];
+        const int fnx = Lf.nx + 1, fny = Lf.ny + 1, nn = (int)Lf.nn;
+        off -= 3 * nn;
+        double* y = x + 3 * Lc.nn;
+        for (int i = threadIdx.x; i < 3 * nn; i += TAIL_THREADS) {
+            const int c = i / nn, n = i - c * nn;
+            const ProlongAt P(Lc, 2, n % fnx, (n / fnx) % fny, n / (fnx * fny));
+            const double v = smooth(w, r[off + i], Lf.diag[i], P(x + c * Lc.nn), (Lf.mask[n] >> c) & 1);
+            if (l > 0) y[i] = v;
+            else L0.x[i] = v;
+        }
+        __syncthreads();
+        x = y;
+    }
+    if (T.n == 1)
+        for (int i = threadIdx.x; i < 3 * nL; i += TAIL_THREADS) L0.x[i] = x[i];
 }
 
 inline unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -578,20 +684,23 @@ void launch_mask_restrict(const MgLevel& Lc, const MgLevel& Lf, cudaStream_t s) 
 void launch_diag_coarsen(const MgLevel& Lc, const MgLevel& Lf, cudaStream_t s) {
     k_diag_coarsen<<<blocks_for(Lc.nn, 128), 128, 0, s>>>(Lc, Lf);
 }
-void launch_restrict(const MgLevel& Lc, const MgLevel& Lf, const double* rf, double* rc, double* a1, double* a2,
+// span 4 (the first transition): x pass, then the y-z pass; span 2: the whole window.  A separate y pass reads
+// less, and its two launches cost more up to about 10^5 coarse nodes.
+void launch_restrict(const MgLevel& Lc, const MgLevel& Lf, const double* rf, double* rc, double* a1,
                      const PcgScalars* S, cudaStream_t s, bool normalize, double* x0, double w) {
+    const dim3 b(blocks_for(Lc.nn, 128), 3);
+    if (Lc.span == 2) {
+        k_restrict_xyz2<<<b, 128, 0, s>>>(Lc, Lf, rf, rc, S, normalize ? 1 : 0, x0, w);
+        return;
+    }
     const int64_t n1 = (int64_t)(Lf.nz + 1) * (Lf.ny + 1) * (Lc.nx + 1);
-    const int64_t n2 = (int64_t)(Lf.nz + 1) * (Lc.ny + 1) * (Lc.nx + 1);
     k_restrict_x<<<blocks_for(n1, 256), 256, 0, s>>>(Lc, Lf, rf, a1, S);
-    k_restrict_y<<<blocks_for(n2, 256), 256, 0, s>>>(Lc, Lf, a1, a2, S);
-    k_restrict_z<<<blocks_for(Lc.nn, 128), 128, 0, s>>>(Lc, Lf, a2, rc, S, normalize ? 1 : 0, x0, w);
+    k_restrict_yz<4><<<b, 128, 0, s>>>(Lc, Lf, a1, rc, S, normalize ? 1 : 0, x0, w);
 }
-void launch_coarse_jacobi(const MgLevel& L, const PcgScalars* S, cudaStream_t s) {
-    k_coarse_jacobi<<<blocks_for(L.nn, 128), 128, 0, s>>>(L, S);
-}
+int restrict_launches(const MgLevel& Lc) { return Lc.span == 2 ? 1 : 2; }
 void launch_prolong_smooth(const MgLevel& Lc, const MgLevel& Lf, const double* xc, const double* rf, double* xf,
                            double weight, const PcgScalars* S, cudaStream_t s) {
-    k_prolong_smooth<<<blocks_for(Lf.nn, 256), 256, 0, s>>>(Lc, Lf, xc, rf, xf, weight, S);
+    k_prolong_smooth<<<dim3(blocks_for(Lf.nn, 128), 3), 128, 0, s>>>(Lc, Lf, xc, rf, xf, weight, S);
 }
 void launch_prolong_smooth0(const MgLevel& Lc, const MgLevel& Lf, const double* xc, const double* r, double* z,
                             double weight, RedSlot dot, PcgScalars* S, cudaStream_t s) {
@@ -637,9 +746,37 @@ void launch_coarse_inverse(const double* LT, const double* Lrow, int N, const in
 }
 void launch_coarse_solve(const MgLevel& L, const double* X, int N, const int* status, const PcgScalars* S,
                          cudaStream_t s) {
-    const int64_t work = N > 0 ? N : L.nn;
-    const unsigned blocks = (unsigned)std::max<int64_t>(1, (work + 127) / 128);
-    k_coarse_solve<<<blocks, 128, (size_t)std::max(N, 1) * sizeof(double), s>>>(L, X, N, status, S);
+    const unsigned blocks = N > 0 ? blocks_for(N, 32) : blocks_for(3 * L.nn, CS_THREADS);
+    const size_t smem = (size_t)(std::max(N, 0) + 32 * CS_ROWS) * sizeof(double);   // N <= 1000: at most 72 KB
+    k_coarse_solve<<<blocks, CS_THREADS, smem, s>>>(L, X, N, status, S);
+}
+cudaError_t mg_kernel_attributes() {
+    const cudaError_t e = cudaFuncSetAttribute(k_coarse_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)((INV_MAX_N + 32 * CS_ROWS) * sizeof(double)));
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k_adapted_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, TAIL_SMEM);
+}
+static size_t tail_smem(const MgLevel* lv, int nlev, int first, int N) {
+    int64_t doubles = (((int64_t)N * N + 1) & ~1ll) + N;
+    for (int l = first; l < nlev; ++l) doubles += 6 * lv[l].nn;
+    return (size_t)doubles * sizeof(double);
+}
+int adapted_tail_first(const MgLevel* lv, int nlev, int N) {
+    if (N > TAIL_N) return nlev;
+    int first = nlev;
+    for (int l = nlev - 1; l >= 1 && lv[l].nn <= TAIL_NODES && (l == nlev - 1 || lv[l + 1].span == 2) &&
+                           tail_smem(lv, nlev, l, N) <= TAIL_SMEM;
+         --l)
+        first = l;
+    // a Jacobi coarsest level alone is better spread
+    return first < nlev - 1 || (first == nlev - 1 && N > 0) ? first : nlev;
+}
+void launch_adapted_tail(const MgLevel* lv, int nlev, int first, const double* X, int N, const int* status, double w,
+                         const PcgScalars* S, cudaStream_t s) {
+    TailLevels T{};
+    T.n = nlev - first;
+    for (int l = first; l < nlev; ++l) T.lv[l - first] = lv[l];
+    k_adapted_tail<<<1, TAIL_THREADS, tail_smem(lv, nlev, first, N), s>>>(T, X, N, status, w, S);
 }
 
 }  // namespace t3d

@@ -203,57 +203,55 @@ __device__ __forceinline__ float hat_sum(int c, int n) {
     return sw;
 }
 
-// a coarse node's restricted residual, masked, and with x0 the Standard cycle's Jacobi start x0 = w0 rc / D
-__device__ __forceinline__ void restrict_store32(const MgLevel32& Lc, int n, float v0, float v1, float v2,
-                                                 float* __restrict__ rc, float* __restrict__ x0, float w0) {
-    const int m = Lc.mask[n];
-    const float v[3] = {(m & 1) ? 0.0f : v0, (m & 2) ? 0.0f : v1, (m & 4) ? 0.0f : v2};
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const int64_t i = c * Lc.nn + n;
-        rc[i] = v[c];
-        if (x0) x0[i] = ((m >> c) & 1) ? 0.0f : (w0 * v[c]) * Lc.diag[i];
-    }
+// component c of a coarse node's restricted residual: the normalised average (transfers.cpp:520-528) or, for the
+// Standard cycle, the transposed prolongation; masked; with x0 the Standard cycle's Jacobi start x0 = w0 rc / D
+template <int SP>
+__device__ __forceinline__ void restrict_store32(const MgLevel32& Lc, const MgLevel32& Lf, int n, int c, int cx, int cy,
+                                                 int cz, float v, int normalize, float* __restrict__ rc,
+                                                 float* __restrict__ x0, float w0) {
+    const float iw = normalize ? 1.0f / (hat_sum<SP>(cz, Lf.nz + 1) * hat_sum<SP>(cy, Lf.ny + 1) *
+                                         hat_sum<SP>(cx, Lf.nx + 1))
+                               : 1.0f;
+    const bool fixed = (Lc.mask[n] >> c) & 1;
+    const float o = fixed ? 0.0f : v * iw;
+    const int64_t i = c * Lc.nn + n;
+    rc[i] = o;
+    if (x0) x0[i] = fixed ? 0.0f : (w0 * o) * Lc.diag[i];
 }
 
-// y and z window sums of the x-pass result a1[fz][fy][cx] in one pass, normalised by the summed in-range
-// weights and masked (the k_restrict_y32 + k_restrict_z32 pair fused; one thread per coarse node).
+// The transfers below take one thread per coarse node and component (component-major); points outside the grid load
+// nothing and add +0, which changes no sum, so that all loads of a window row are in flight together.
+// y and z window sums of the x-pass result a1[fz][fy][cx] in one pass.
 template <int SP>
 __device__ __forceinline__ void restrict_yz32(VB vb, const MgLevel32& Lc, const MgLevel32& Lf,
                                               const float* __restrict__ a1, float* __restrict__ rc,
                                               const PcgScalars* S, int normalize, float* __restrict__ x0, float w0) {
     if (S->done) return;
     constexpr int WS = 2 * SP - 1;
-    const int n = vb.b * blockDim.x + threadIdx.x;
-    if (n >= Lc.nn) return;
+    const int i = vb.b * blockDim.x + threadIdx.x, nn = (int)Lc.nn;
+    if (i >= 3 * nn) return;
+    const int c = i / nn, n = i - c * nn;
     const int cnx = Lc.nx + 1, cny = Lc.ny + 1;
-    const int fnx = Lf.nx + 1, fny = Lf.ny + 1, fnz = Lf.nz + 1;
+    const int fny = Lf.ny + 1, fnz = Lf.nz + 1;
     const int cx = n % cnx, cy = (n / cnx) % cny, cz = n / (cnx * cny);
-    const int total1 = fnz * fny * cnx;
-    float v0 = 0.0f, v1 = 0.0f, v2 = 0.0f;
+    const float* __restrict__ a = a1 + (int64_t)c * fnz * fny * cnx + cx;
+    float v = 0.0f;
 #pragma unroll
     for (int iz = 0; iz < WS; ++iz) {
         const int fz = cz * SP + iz - (SP - 1);
-        if (fz < 0 || fz >= fnz) continue;
-        float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f;
+        const bool zin = fz >= 0 && fz < fnz;
+        float q[WS];
 #pragma unroll
         for (int iy = 0; iy < WS; ++iy) {
             const int fy = cy * SP + iy - (SP - 1);
-            if (fy < 0 || fy >= fny) continue;
-            const float w = hatf(iy, SP);
-            const int i = (fz * fny + fy) * cnx + cx;
-            s0 = fmaf(w, a1[i], s0);
-            s1 = fmaf(w, a1[total1 + i], s1);
-            s2 = fmaf(w, a1[2 * total1 + i], s2);
+            q[iy] = zin && fy >= 0 && fy < fny ? a[(fz * fny + fy) * cnx] : 0.0f;
         }
-        const float w = hatf(iz, SP);
-        v0 = fmaf(w, s0, v0);
-        v1 = fmaf(w, s1, v1);
-        v2 = fmaf(w, s2, v2);
+        float t = 0.0f;
+#pragma unroll
+        for (int iy = 0; iy < WS; ++iy) t = fmaf(hatf(iy, SP), q[iy], t);
+        v = fmaf(hatf(iz, SP), t, v);
     }
-    // normalised average (transfers.cpp:520-528) or, for the Standard cycle, the transposed prolongation
-    const float iw = normalize ? 1.0f / (hat_sum<SP>(cz, fnz) * hat_sum<SP>(cy, fny) * hat_sum<SP>(cx, fnx)) : 1.0f;
-    restrict_store32(Lc, n, v0 * iw, v1 * iw, v2 * iw, rc, x0, w0);
+    restrict_store32<SP>(Lc, Lf, n, c, cx, cy, cz, v, normalize, rc, x0, w0);
 }
 template <int SP>
 __global__ void __launch_bounds__(256) k_restrict_yz32(MgLevel32 Lc, MgLevel32 Lf, const float* __restrict__ a1,
@@ -269,46 +267,35 @@ __device__ __forceinline__ void restrict_xyz32(VB vb, const MgLevel32& Lc, const
                                                const PcgScalars* S, int normalize, float* __restrict__ x0, float w0) {
     if (S->done) return;
     constexpr int WS = 2 * SP - 1;
-    const int n = vb.b * blockDim.x + threadIdx.x;
-    if (n >= Lc.nn) return;
+    const int i = vb.b * blockDim.x + threadIdx.x, nn = (int)Lc.nn;
+    if (i >= 3 * nn) return;
+    const int c = i / nn, n = i - c * nn;
     const int cnx = Lc.nx + 1, cny = Lc.ny + 1;
     const int fnx = Lf.nx + 1, fny = Lf.ny + 1, fnz = Lf.nz + 1;
     const int cx = n % cnx, cy = (n / cnx) % cny, cz = n / (cnx * cny);
-    const int fNN = (int)Lf.cs;
-    float v0 = 0.0f, v1 = 0.0f, v2 = 0.0f;
+    const float* __restrict__ r = rf + c * Lf.cs;
+    float q[WS * WS * WS];
+#pragma unroll
+    for (int k = 0; k < WS * WS * WS; ++k) {
+        const int fx = cx * SP + k % WS - (SP - 1), fy = cy * SP + (k / WS) % WS - (SP - 1),
+                  fz = cz * SP + k / (WS * WS) - (SP - 1);
+        const bool in = fx >= 0 && fx < fnx && fy >= 0 && fy < fny && fz >= 0 && fz < fnz;
+        q[k] = in ? r[(fz * fny + fy) * Lf.pitch + fx] : 0.0f;
+    }
+    float v = 0.0f;
 #pragma unroll
     for (int iz = 0; iz < WS; ++iz) {
-        const int fz = cz * SP + iz - (SP - 1);
-        if (fz < 0 || fz >= fnz) continue;
-        float t0 = 0.0f, t1 = 0.0f, t2 = 0.0f;
+        float t = 0.0f;
 #pragma unroll
         for (int iy = 0; iy < WS; ++iy) {
-            const int fy = cy * SP + iy - (SP - 1);
-            if (fy < 0 || fy >= fny) continue;
-            const float* __restrict__ src = rf + (fz * fny + fy) * Lf.pitch;
-            float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f;
+            float p = 0.0f;
 #pragma unroll
-            for (int ix = 0; ix < WS; ++ix) {
-                const int fx = cx * SP + ix - (SP - 1);
-                if (fx < 0 || fx >= fnx) continue;
-                const float w = hatf(ix, SP);
-                s0 = fmaf(w, src[fx], s0);
-                s1 = fmaf(w, src[fNN + fx], s1);
-                s2 = fmaf(w, src[2 * fNN + fx], s2);
-            }
-            const float w = hatf(iy, SP);
-            t0 = fmaf(w, s0, t0);
-            t1 = fmaf(w, s1, t1);
-            t2 = fmaf(w, s2, t2);
+            for (int ix = 0; ix < WS; ++ix) p = fmaf(hatf(ix, SP), q[(iz * WS + iy) * WS + ix], p);
+            t = fmaf(hatf(iy, SP), p, t);
         }
-        const float w = hatf(iz, SP);
-        v0 = fmaf(w, t0, v0);
-        v1 = fmaf(w, t1, v1);
-        v2 = fmaf(w, t2, v2);
+        v = fmaf(hatf(iz, SP), t, v);
     }
-    // normalised average (transfers.cpp:520-528) or, for the Standard cycle, the transposed prolongation
-    const float iw = normalize ? 1.0f / (hat_sum<SP>(cz, fnz) * hat_sum<SP>(cy, fny) * hat_sum<SP>(cx, fnx)) : 1.0f;
-    restrict_store32(Lc, n, v0 * iw, v1 * iw, v2 * iw, rc, x0, w0);
+    restrict_store32<SP>(Lc, Lf, n, c, cx, cy, cz, v, normalize, rc, x0, w0);
 }
 template <int SP>
 __global__ void __launch_bounds__(256) k_restrict_xyz32(MgLevel32 Lc, MgLevel32 Lf, const float* __restrict__ rf,
@@ -477,8 +464,17 @@ __device__ __forceinline__ void coarse_solve32(VB vb, const MgLevel32& L, const 
     const int i = vb.b * 32 + lane;
     const int per = (N + COARSE_WARPS - 1) / COARSE_WARPS, j0 = w * per, j1 = min(N, j0 + per);
     double acc = 0.0;
-    if (i < N)
-        for (int j = j0; j < j1; ++j) acc = fma(X[(int64_t)j * N + i], rs[j], acc);
+    if (i < N) {
+        int j = j0;
+        for (; j + 16 <= j1; j += 16) {   // 16 loads in flight ahead of the chain
+            double q[16];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) q[k] = X[(int64_t)(j + k) * N + i];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) acc = fma(q[k], rs[j + k], acc);
+        }
+        for (; j < j1; ++j) acc = fma(X[(int64_t)j * N + i], rs[j], acc);
+    }
     part[w * 32 + lane] = acc;
     __syncthreads();
     if (w == 0 && i < N) {
@@ -683,9 +679,9 @@ int batch_blocks_restrict(const BatchRestrict& a, int stage) {
     const MgLevel32& Lf = a.Lf;
     if (Lc.span == 4) {
         if (stage == 0) return (int)blocks_for((int64_t)(Lf.nz + 1) * (Lf.ny + 1) * (Lc.nx + 1), 256);
-        return (int)blocks_for(Lc.nn, 256);
+        return (int)blocks_for(3 * Lc.nn, 256);
     }
-    return stage == 0 ? (int)blocks_for(Lc.nn, 256) : 0;
+    return stage == 0 ? (int)blocks_for(3 * Lc.nn, 256) : 0;
 }
 int batch_blocks_prolong(const BatchProlong& a) { return (int)blocks_for(a.Lf.nn, 256); }
 int batch_blocks_coarse(const BatchCoarse& a) { return std::max(1, coarse_blocks(a.N, a.L.nn)); }
@@ -747,9 +743,9 @@ void launch_restrict32(const MgLevel32& Lc, const MgLevel32& Lf, const float* rf
     const int64_t n1 = (int64_t)(Lf.nz + 1) * (Lf.ny + 1) * (Lc.nx + 1);
     if (Lc.span == 4) {
         k_restrict_x32<<<blocks_for(n1, 256), 256, 0, s>>>(Lc, Lf, rf, a1, S);
-        k_restrict_yz32<4><<<blocks_for(Lc.nn, 256), 256, 0, s>>>(Lc, Lf, a1, rc, S, normalize ? 1 : 0, x0, w);
+        k_restrict_yz32<4><<<blocks_for(3 * Lc.nn, 256), 256, 0, s>>>(Lc, Lf, a1, rc, S, normalize ? 1 : 0, x0, w);
     } else {
-        k_restrict_xyz32<2><<<blocks_for(Lc.nn, 256), 256, 0, s>>>(Lc, Lf, rf, rc, S, normalize ? 1 : 0, x0, w);
+        k_restrict_xyz32<2><<<blocks_for(3 * Lc.nn, 256), 256, 0, s>>>(Lc, Lf, rf, rc, S, normalize ? 1 : 0, x0, w);
     }
 }
 void launch_rows_to32(int64_t rows, int len, const double* a, float* b, cudaStream_t s) {

@@ -111,10 +111,9 @@ void launch_mask_restrict(const MgLevel& Lc, const MgLevel& Lf, cudaStream_t s);
 void launch_diag_coarsen(const MgLevel& Lc, const MgLevel& Lf, cudaStream_t s);
 // separable restriction; a1, a2: pass buffers of 3*(fnz*fny*cnx) and 3*(fnz*cny*cnx) doubles
 // normalize = false: the transpose of the trilinear prolongation (no division by the weight sum)
-void launch_restrict(const MgLevel& Lc, const MgLevel& Lf, const double* rf, double* rc, double* a1, double* a2,
+void launch_restrict(const MgLevel& Lc, const MgLevel& Lf, const double* rf, double* rc, double* a1,
                      const PcgScalars* S, cudaStream_t s, bool normalize = true,
                      double* x0 = nullptr, double w = 0.0);
-void launch_coarse_jacobi(const MgLevel& L, const PcgScalars* S, cudaStream_t s);
 void launch_prolong_smooth(const MgLevel& Lc, const MgLevel& Lf, const double* xc, const double* rf, double* xf,
                            double weight, const PcgScalars* S, cudaStream_t s);
 void launch_prolong_smooth0(const MgLevel& Lc, const MgLevel& Lf, const double* xc, const double* r, double* z,
@@ -131,6 +130,14 @@ int launch_cholesky(const double* A, double* LT, double* Lrow, int N, int* statu
 // *status != 1, preconditioner.cpp:76-77, 195-215)
 void launch_coarse_inverse(const double* LT, const double* Lrow, int N, const int* status, double* X,
                            cudaStream_t s);
+// shared-memory limits of the V-cycle kernels (per function: their bounds, the same for every context)
+cudaError_t mg_kernel_attributes();
+int restrict_launches(const MgLevel& Lc);
+// The Adapted cycle from level `first` down and back in one kernel: lv[first].r -> lv[first].x.  adapted_tail_first:
+// the finest level it takes (nlev: none; then the levels run in separate kernels).
+int adapted_tail_first(const MgLevel* lv, int nlev, int N);
+void launch_adapted_tail(const MgLevel* lv, int nlev, int first, const double* X, int N, const int* status, double w,
+                         const PcgScalars* S, cudaStream_t s);
 void launch_coarse_solve(const MgLevel& L, const double* X, int N, const int* status, const PcgScalars* S,
                          cudaStream_t s);
 
