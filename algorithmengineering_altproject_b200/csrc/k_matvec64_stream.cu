@@ -20,6 +20,11 @@
 // modifier); the 24 rows of a column run in ke_row_order so that consecutive DFMAs share a coefficient
 // register.  Any other Ke (t3d_set_ke) is passed by value and read from the constant bank.
 // p.Ap is not fused: the caller folds it in the canonical order.
+// What bounds it: the chains are 576 DFMAs a thread and layer, 1.3 ms at 256x512x256 with the tile halo; the rest of a
+// layer used to be as many instructions again (index divisions in the loads, corner and side arithmetic in the fold:
+// FP64 pipe 49 % busy, issue slots 49 %), which did not overlap them.  With the loads' places fixed per thread and the
+// fold's order reduced to three parity bits the launch takes 2.33 ms instead of 2.81 (96x192x96: 0.183 -> 0.155 with
+// its dot, 48x96x48 44 -> 36 us).
 #include <algorithm>
 #include <cmath>
 
@@ -63,29 +68,49 @@ __device__ __forceinline__ unsigned smem_addr(const double* p) {
     return (unsigned)__cvta_generic_to_shared(p);
 }
 
-// footprint of node plane iz, (PX x PY) nodes from (X0-1, Y0-1), 3 components, zero outside the grid
-__device__ __forceinline__ void load_plane(const Grid& g, const double* __restrict__ u, int X0, int Y0, int iz,
-                                           double* dst) {
-    constexpr int AREA = S64::PY * S64::PX;
-    const bool zok = iz >= 0 && iz < g.nnz;
-    for (int i = threadIdx.x; i < 3 * AREA; i += S64::NT) {
-        const int c = i / AREA, rem = i - c * AREA, py = rem / S64::PX, px = rem - py * S64::PX;
-        const int ix = X0 - 1 + px, iy = Y0 - 1 + py;
-        const bool ok = zok && ix >= 0 && ix < g.nnx && iy >= 0 && iy < g.nny;
-        const double* src = ok ? u + c * g.NN + g.node(ix, iy, iz) : u;
-        cp_async8(smem_addr(dst + i), src, ok);
+// One thread's share of a tile's loads: its own node of the (PX x PY) footprint from (X0-1, Y0-1), one node of the
+// last row (warp 0) or column (the first PY threads of warp 1), and the modulus of its element column from cell
+// (X0-1, Y0-1).  Places outside the grid load zero; cells beyond the ghost ring too (they are skipped like ghosts).
+// The offsets in a plane are fixed for the item, so a step costs an address and a copy per value.
+struct S64Loads {
+    int off, off2;        // node offsets within a plane of u; the second for warps 0 and 1
+    int dst2;             // the second node's place in the footprint
+    bool ok, ok2, have2;  // inside the grid; a second node at all
+    int eoff;             // cell offset within a layer (ghost ring included)
+    bool eok;
+    __device__ __forceinline__ S64Loads(const Grid& g, int X0, int Y0) {
+        const int tx = threadIdx.x % S64::BX, ty = threadIdx.x / S64::BX;
+        const int ix = X0 - 1 + tx, iy = Y0 - 1 + ty;
+        ok = ix >= 0 && ix < g.nnx && iy >= 0 && iy < g.nny;
+        off = ok ? iy * g.nnx + ix : 0;
+        const int px = ty == 0 ? tx : S64::BX, py = ty == 0 ? S64::BY : tx;
+        have2 = ty == 0 || (ty == 1 && tx < S64::PY);
+        const int jx = X0 - 1 + px, jy = Y0 - 1 + py;
+        ok2 = jx >= 0 && jx < g.nnx && jy >= 0 && jy < g.nny;
+        off2 = ok2 ? jy * g.nnx + jx : 0;
+        dst2 = py * S64::PX + px;
+        eok = ix <= g.nx && iy <= g.ny;
+        eoff = eok ? (iy + 1) * g.ex + ix + 1 : 0;
     }
-}
-
-// E of element layer cz over the tile's BX x BY element columns from cell (X0-1, Y0-1); cells beyond
-// the ghost ring read as 0 (they are skipped like the ghosts)
-__device__ __forceinline__ void load_emod(const Grid& g, const double* __restrict__ E, int X0, int Y0, int cz,
-                                          double* dst) {
-    const int tx = threadIdx.x % S64::BX, ty = threadIdx.x / S64::BX;
-    const int cx = X0 - 1 + tx, cy = Y0 - 1 + ty;
-    const bool ok = cx <= g.nx && cy <= g.ny;
-    cp_async8(smem_addr(dst + threadIdx.x), ok ? E + g.cell(cx, cy, cz) : E, ok);
-}
+    __device__ __forceinline__ void plane(const Grid& g, const double* __restrict__ u, int iz, double* dst) const {
+        constexpr int AREA = S64::PY * S64::PX;
+        const bool zok = iz >= 0 && iz < g.nnz;
+        const double* src = u + (zok ? (int64_t)iz * g.nnx * g.nny : 0);
+        const int tx = threadIdx.x % S64::BX, ty = threadIdx.x / S64::BX;
+        const unsigned d = smem_addr(dst + ty * S64::PX + tx);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) cp_async8(d + c * AREA * 8, src + c * g.NN + off, zok && ok);
+        if (have2) {
+            const unsigned d2 = smem_addr(dst + dst2);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) cp_async8(d2 + c * AREA * 8, src + c * g.NN + off2, zok && ok2);
+        }
+    }
+    __device__ __forceinline__ void emod(const Grid& g, const double* __restrict__ E, int cz, double* dst) const {
+        cp_async8(smem_addr(dst + threadIdx.x), E + (eok ? (int64_t)(cz + 1) * g.ex * g.ey : 0) + eoff, eok);
+    }
+};
+static_assert(S64_BX == 32 && S64_BY >= 2 && S64::PY <= 32, "S64Loads: warps 0 and 1 take the last row and column");
 
 template <bool PAT>
 __global__ void __launch_bounds__(S64::NT, 2) k_matvec64_stream(Grid g, Stream64Tiling t, const Ke64 ke,
@@ -110,10 +135,11 @@ __global__ void __launch_bounds__(S64::NT, 2) k_matvec64_stream(Grid g, Stream64
         const int X0 = tix * (BX - 1), Y0 = tiy * (BY - 1);
         const int Z0 = sl * t.slab, Z1 = min(Z0 + t.slab, g.nnz);
         const int nlay = Z1 - Z0 + 1;   // element layers Z0-1 .. Z1-1
+        const S64Loads ld(g, X0, Y0);
         __syncthreads();                // the previous item's owners are done with the rings
-        load_plane(g, u, X0, Y0, Z0 - 1, sm + S64::PLANE);
-        load_plane(g, u, X0, Y0, Z0, sm + S64::PLANE + S64::PLANE_SZ);
-        load_emod(g, E, X0, Y0, Z0 - 1, sm + S64::EMOD);
+        ld.plane(g, u, Z0 - 1, sm + S64::PLANE);
+        ld.plane(g, u, Z0, sm + S64::PLANE + S64::PLANE_SZ);
+        ld.emod(g, E, Z0 - 1, sm + S64::EMOD);
         cp_commit();
 #pragma unroll 1
         for (int k = 0; k < nlay; ++k) {
@@ -121,8 +147,8 @@ __global__ void __launch_bounds__(S64::NT, 2) k_matvec64_stream(Grid g, Stream64
             cp_wait0();
             __syncthreads();
             if (k + 1 < nlay) {          // node plane cz+2 and the E of layer cz+1 for the next step
-                load_plane(g, u, X0, Y0, cz + 2, sm + S64::PLANE + ((k + 2) % 3) * S64::PLANE_SZ);
-                load_emod(g, E, X0, Y0, cz + 1, sm + S64::EMOD + ((k + 1) % 3) * NT);
+                ld.plane(g, u, cz + 2, sm + S64::PLANE + ((k + 2) % 3) * S64::PLANE_SZ);
+                ld.emod(g, E, cz + 1, sm + S64::EMOD + ((k + 1) % 3) * NT);
             }
             cp_commit();
             // ---- element (tx, ty) of layer cz: the 24 FMA chains f_row = fma(Ke[row][j], u_e[j], f_row), j = 0..23
@@ -182,19 +208,27 @@ __global__ void __launch_bounds__(S64::NT, 2) k_matvec64_stream(Grid g, Stream64
                     const double* Eabove = sm + S64::EMOD + (k % 3) * NT;
                     const double* Fbelow = sm + S64::FT + ((k - 1) & 1) * 12 * NT;
                     double y0 = 0.0, y1 = 0.0, y2 = 0.0;
+                    // the node's colour order: bit 0, 1, 2 of the colour choose the element's side in x, y, z, the even
+                    // one first; element column tx + sx (cx = ix-1+sx), row ty + sy, layer iz-1 (sz = 0) or iz
+                    const int fx = (ix - 1) & 1, fy = (g.ny - iy) & 1, fz = (iz - 1) & 1;
 #pragma unroll
-                    for (int col = 0; col < 8; ++col) {
-                        const int sx = (((ix - 1) & 1) == (col & 1)) ? 0 : 1;   // element column tx+sx: cx = ix-1+sx
-                        const int sy = (((g.ny - iy) & 1) == ((col >> 1) & 1)) ? 0 : 1;
-                        const int sz = (((iz - 1) & 1) == ((col >> 2) & 1)) ? 0 : 1;   // 0: layer iz-1, 1: layer iz
-                        const int e = (ty + sy) * BX + tx + sx;
-                        const double Ec = sz ? Eabove[e] : Ebelow[e];
-                        if (Ec <= 1.0e-16) continue;
-                        const int a = corner_of(1 - sx, 1 - sy, 1 - sz);
-                        const double* F = sz ? Fb + 3 * a * NT : Fbelow + 3 * (a - 4) * NT;
-                        y0 = fma(F[e], Ec, y0);
-                        y1 = fma(F[NT + e], Ec, y1);
-                        y2 = fma(F[2 * NT + e], Ec, y2);
+                    for (int h = 0; h < 2; ++h) {
+                        const int sz = h ^ fz;   // the same for the whole block
+                        const double* Em = sz ? Eabove : Ebelow;
+                        const double* Fm = sz ? Fb : Fbelow;
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const int sx = (q & 1) ^ fx, sy = (q >> 1) ^ fy;
+                            const int e = threadIdx.x + sy * BX + sx;
+                            const double Ec = Em[e];
+                            if (Ec <= 1.0e-16) continue;
+                            // corner of the element in its layer's plane: 1 - sx, 1 - sy -> 0 (0,1), 1 (1,1), 2 (1,0), 3 (0,0)
+                            const int a = sy ? 3 - (1 - sx) : 1 - sx;
+                            const double* F = Fm + 3 * a * NT + e;
+                            y0 = fma(F[0], Ec, y0);
+                            y1 = fma(F[NT], Ec, y1);
+                            y2 = fma(F[2 * NT], Ec, y2);
+                        }
                     }
                     const int64_t n = g.node(ix, iy, iz);
                     const int mk = mask[n];
