@@ -68,7 +68,7 @@ struct Batch {
     ModalKe kh{};
     std::vector<void*> dallocs;
     bool standard = false;       // the members' V-cycle (all the same): Standard, else Adapted
-    LaunchList mv, up, dir, p0, co, mv1, mv2, jac;
+    LaunchList mv, up, dir, p0, co, mv1, mv2;
     LaunchList rs0[8], rs1[8], pr[8], lop[8], pa[8];
     int maxL = 0, coarse_max = 0;
     CUtensorMap* maps = nullptr;
@@ -124,7 +124,7 @@ struct Batch {
         dS = nullptr;
         dflags = nullptr;
         err = nullptr;
-        mv = up = dir = p0 = co = mv1 = mv2 = jac = LaunchList{};
+        mv = up = dir = p0 = co = mv1 = mv2 = LaunchList{};
         for (int l = 0; l < 8; ++l) rs0[l] = rs1[l] = pr[l] = lop[l] = pa[l] = LaunchList{};
     }
 
@@ -255,7 +255,8 @@ static int batch_lists(Batch* B) {
         return BatchMatvec{c->g, c->mt, c->mask0, c->Ap32, c->slot[0], c->S32, q, q + 1, nullptr, nullptr, 0.f};
     }, mvb));
     CHECK(list(&B->up, all, [](t3d_context* c, int) {
-        return BatchUpdate{c->g.NNp, c->r32, c->Ap32, c->slot[1], c->S32};
+        return BatchUpdate{c->g.NNp, c->r32, c->Ap32, c->slot[1], c->S32, c->lv32[0].diag,
+                           c->standard ? c->z32 : nullptr, c->prm.mg_standard_weight};
     }, [](const BatchUpdate& a) { return batch_blocks_update(a.NNp); }));
     CHECK(list(&B->dir, all, [](t3d_context* c, int) {
         return BatchDirection{c->g.NNp, c->z32, c->p32, c->d32, c->S32};
@@ -300,11 +301,6 @@ static int batch_lists(Batch* B) {
             B->iter_kernels += 1;
             B->iter_blocks += B->lop[l].blocks;
         }
-    }
-    if (B->standard) {
-        CHECK(list(&B->jac, all, [](t3d_context* c, int) {
-            return BatchJacobi{c->lv32[0], c->r32, c->z32, c->prm.mg_standard_weight, c->S32};
-        }, [](const BatchJacobi& a) { return batch_blocks_jacobi(a); }));
     }
     if (B->standard) {
         CHECK(list(&B->mv1, all, [&](t3d_context* c, int i) {
@@ -401,7 +397,7 @@ static void batch_product(Batch* B, int mode, const LaunchList& L) {
 }
 
 // vcycle32 (context.cu) for every member: the Adapted cycle, or the Standard one (vcycle32_standard) with its
-// level-0 residual and correction fused into the TMA products
+// level-0 residual and correction fused into the TMA products and its start z = w r / D into the update before
 static void batch_vcycle(Batch* B) {
     if (!B->standard) {
         for (int l = 0; l + 1 < B->maxL; ++l) batch_restrict(B, l);
@@ -411,7 +407,6 @@ static void batch_vcycle(Batch* B) {
         launch_batch_prolong0_32(args_of<BatchProlong0>(B->p0), B->p0.act, B->p0.n, B->st);
         return;
     }
-    launch_batch_jacobi32(args_of<BatchJacobi>(B->jac), B->jac.act, B->jac.n, B->st);        // z = w r / D
     for (int l = 0; l + 1 < B->maxL; ++l) {
         const LaunchList& op = B->lop[l];
         if (l == 0) batch_product(B, 1, B->mv1);                                                     // t = r - K x

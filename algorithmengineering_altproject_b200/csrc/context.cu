@@ -799,7 +799,8 @@ static int pcg_solve(Context* c, double tol, int maxit, int* iters) {
 // ------------------------------------------------------------------ mixed-precision solve
 // The Standard cycle in FP32 (k_mg_standard32.cu): the same steps as vcycle_standard; level 0 uses Ap32 as
 // scratch and the modal FP32 K(E) of the hierarchy's moduli as its operator
-static void vcycle32_standard(Context* c, const float* r, float* z, PcgScalars* S, RedSlot dot) {
+// started: z already holds the level-0 start w r / D (the PCG update writes it)
+static void vcycle32_standard(Context* c, const float* r, float* z, PcgScalars* S, RedSlot dot, bool started) {
     const int L = c->nlev;
     const float w = c->prm.mg_standard_weight;
     // level 0 with the modal TMA kernel: the residual and the correction (with r.z) run in its epilogue
@@ -807,8 +808,8 @@ static void vcycle32_standard(Context* c, const float* r, float* z, PcgScalars* 
     auto product0 = [&](const float* x, float* y) {
         matvec32(c, x, y, RedSlot{nullptr, nullptr}, S, 0, c->E_mg32);
     };
-    launch_jacobi_init32(c->lv32[0], r, z, w, S, c->st);
-    c->launches += 2;
+    if (!started) launch_jacobi_init32(c->lv32[0], r, z, w, S, c->st);
+    c->launches += started ? 1 : 2;
     if (fuse) {
         launch_matvec32_fused(1, c->g, c->kh, c->mt, c->E_mg32, c->mask0, z, c->Ap32, r, nullptr, w,
                               RedSlot{nullptr, nullptr}, S, c->tma_err, c->st);
@@ -850,9 +851,9 @@ static void vcycle32_standard(Context* c, const float* r, float* z, PcgScalars* 
     c->launches += 3;
 }
 
-static void vcycle32(Context* c, const float* r, float* z, PcgScalars* S, RedSlot dot) {
+static void vcycle32(Context* c, const float* r, float* z, PcgScalars* S, RedSlot dot, bool started = false) {
     if (c->standard) {
-        vcycle32_standard(c, r, z, S, dot);
+        vcycle32_standard(c, r, z, S, dot, started);
         return;
     }
     const int L = c->nlev;
@@ -877,8 +878,9 @@ int member_vcycle32(Context* c, const float* r, float* z, PcgScalars* S, RedSlot
 static void pcg32_iteration(Context* c) {
     c->launches += 2;
     matvec32(c, c->p32, c->Ap32, c->slot[0], c->S32);
-    launch_pcg_update32(c->g, c->d32, c->r32, c->p32, c->Ap32, c->slot[1], c->S32, c->st);
-    vcycle32(c, c->r32, c->z32, c->S32, c->slot[2]);
+    launch_pcg_update32(c->g, c->r32, c->Ap32, c->slot[1], c->S32, c->lv32[0].diag, c->standard ? c->z32 : nullptr,
+                        c->prm.mg_standard_weight, c->st);
+    vcycle32(c, c->r32, c->z32, c->S32, c->slot[2], true);
     launch_pcg_direction32(c->g, c->z32, c->p32, c->d32, c->S32, c->st);
 }
 

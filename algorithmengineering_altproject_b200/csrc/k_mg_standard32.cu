@@ -47,15 +47,15 @@ __device__ __forceinline__ float lane_of(const V& v, int k) {
 __device__ __forceinline__ void jacobi_init0_32(VB vb, const MgLevel32& L, const float* __restrict__ r,
                                                float* __restrict__ x, float w) {
     const int fnx = L.nx + 1, q4 = L.pitch >> 2;
-    const int64_t rows = (int64_t)(L.ny + 1) * (L.nz + 1), per_c = rows * q4;
-    for (int64_t t = (int64_t)vb.b * blockDim.x + threadIdx.x; t < 3 * per_c; t += (int64_t)vb.n * blockDim.x) {
-        const int c = (int)(t / per_c);
-        const int64_t rt = t - c * per_c, row = rt / q4;
-        const int x0 = 4 * (int)(rt - row * q4);
-        const int64_t i = c * L.cs + row * L.pitch + x0;
+    const int rows = (L.ny + 1) * (L.nz + 1), per_c = rows * q4;   // 3 per_c < 2^31: the grids' DOFs fit 32 bits
+    for (int t = vb.b * blockDim.x + threadIdx.x; t < 3 * per_c; t += vb.n * blockDim.x) {
+        const int c = t / per_c;
+        const int rt = t - c * per_c, row = rt / q4;
+        const int x0 = 4 * (rt - row * q4);
+        const int64_t i = c * L.cs + (int64_t)row * L.pitch + x0;
         const float4 rv = *reinterpret_cast<const float4*>(r + i), dv = *reinterpret_cast<const float4*>(L.diag + i);
         float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-        const uint8_t* mk = L.mask + row * fnx;
+        const uint8_t* mk = L.mask + (int64_t)row * fnx;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const int fx = x0 + k;
@@ -76,11 +76,11 @@ __device__ __forceinline__ void prolong_add0_32(VB vb, const MgLevel32& Lc, cons
     using V = typename std::conditional<SP == 4, float4, float2>::type;
     const int fnx = Lf.nx + 1, fny = Lf.ny + 1, cnx = Lc.nx + 1, cny = Lc.ny + 1;
     const int runs = Lc.nx + 1;   // Lf.nx = SP Lc.nx: Lc.nx runs of SP nodes and the last node
-    const int64_t total = (int64_t)runs * fny * (Lf.nz + 1);
-    for (int64_t t = (int64_t)vb.b * blockDim.x + threadIdx.x; t < total; t += (int64_t)vb.n * blockDim.x) {
-        const int64_t row = t / runs;
-        const int j = (int)(t - row * runs);
-        const int fz = (int)(row / fny), fy = (int)(row - (int64_t)fz * fny);
+    const int total = runs * fny * (Lf.nz + 1);   // at most the level's nodes
+    for (int t = vb.b * blockDim.x + threadIdx.x; t < total; t += vb.n * blockDim.x) {
+        const int row = t / runs;
+        const int j = t - row * runs;
+        const int fz = row / fny, fy = row - fz * fny;
         const bool last = j == Lc.nx;
         const int cx = last ? Lc.nx - 1 : j;
         int cy = fy / SP, cz = fz / SP;
@@ -88,7 +88,7 @@ __device__ __forceinline__ void prolong_add0_32(VB vb, const MgLevel32& Lc, cons
         if (cz >= Lc.nz) cz = Lc.nz - 1;
         // the run's fine rows are loaded first, so that their HBM reads and the coarse corners' L2 reads are in
         // flight together (xo may be xi: every read of the run precedes its writes, as before)
-        const int64_t rb = row * Lf.pitch + SP * j;
+        const int64_t rb = (int64_t)row * Lf.pitch + SP * j;
         V v[3];
         if (!last) {
 #pragma unroll
@@ -99,8 +99,7 @@ __device__ __forceinline__ void prolong_add0_32(VB vb, const MgLevel32& Lc, cons
         for (int c = 0; c < 3; ++c)
 #pragma unroll
             for (int A = 0; A < 8; ++A)
-                X[c][A] = xc[c * Lc.cs + ((int64_t)(cz + corner_dz(A)) * cny + cy + corner_dy(A)) * cnx + cx +
-                             corner_dx(A)];
+                X[c][A] = xc[c * Lc.cs + ((cz + corner_dz(A)) * cny + cy + corner_dy(A)) * cnx + cx + corner_dx(A)];
         // the weights tri_wf(...) = w_x w_y w_z are products of multiples of 1/SP (SP = 2, 4): exact in any
         // order, so w_y w_z is formed once per run and w_x per node, giving the same values bit for bit
         constexpr float is = 1.0f / (float)SP;
@@ -109,7 +108,7 @@ __device__ __forceinline__ void prolong_add0_32(VB vb, const MgLevel32& Lc, cons
 #pragma unroll
         for (int q = 0; q < 4; ++q)
             wyz[q] = ((q & 1) ? ry * is : (SP - ry) * is) * ((q & 2) ? rz * is : (SP - rz) * is);
-        const uint8_t* mk = Lf.mask + row * fnx;
+        const uint8_t* mk = Lf.mask + (int64_t)row * fnx;
         if (last) {   // x = nx: one node, all weight on the cell's upper x corners
             const int fx = Lf.nx, m = mk[fx];
 #pragma unroll
@@ -118,7 +117,7 @@ __device__ __forceinline__ void prolong_add0_32(VB vb, const MgLevel32& Lc, cons
 #pragma unroll
                 for (int A = 0; A < 8; ++A)
                     p = fmaf((corner_dx(A) ? 1.0f : 0.0f) * wyz[corner_dy(A) + 2 * corner_dz(A)], X[c][A], p);
-                const int64_t i = c * Lf.cs + row * Lf.pitch + fx;
+                const int64_t i = c * Lf.cs + (int64_t)row * Lf.pitch + fx;
                 xo[i] = ((m >> c) & 1) ? 0.0f : xi[i] + p;
             }
             continue;
@@ -221,8 +220,9 @@ __device__ __forceinline__ void prolong_add32(VB vb, const MgLevel32& Lc, const 
     }
     const int s = Lc.span;
     const int fnx = Lf.nx + 1, fny = Lf.ny + 1, cnx = Lc.nx + 1, cny = Lc.ny + 1;
-    for (int64_t n = (int64_t)vb.b * blockDim.x + threadIdx.x; n < Lf.nn; n += (int64_t)vb.n * blockDim.x) {
-        const int fx = (int)(n % fnx), fy = (int)((n / fnx) % fny), fz = (int)(n / ((int64_t)fnx * fny));
+    const int nn = (int)Lf.nn;
+    for (int n = vb.b * blockDim.x + threadIdx.x; n < nn; n += vb.n * blockDim.x) {
+        const int fx = n % fnx, fy = (n / fnx) % fny, fz = n / (fnx * fny);
         int cx = fx / s, cy = fy / s, cz = fz / s;
         if (cx >= Lc.nx) cx = Lc.nx - 1;
         if (cy >= Lc.ny) cy = Lc.ny - 1;
@@ -233,8 +233,7 @@ __device__ __forceinline__ void prolong_add32(VB vb, const MgLevel32& Lc, const 
             float p = 0.0f;
             for (int A = 0; A < 8; ++A)
                 p = fmaf(tri_wf(s, fx - cx * s, fy - cy * s, fz - cz * s, A),
-                         xc[c * Lc.cs + ((int64_t)(cz + corner_dz(A)) * cny + cy + corner_dy(A)) * cnx + cx + corner_dx(A)],
-                         p);
+                         xc[c * Lc.cs + ((cz + corner_dz(A)) * cny + cy + corner_dy(A)) * cnx + cx + corner_dx(A)], p);
             const int64_t i = c * Lf.cs + v;
             xo[i] = ((m >> c) & 1) ? 0.0f : xi[i] + p;
         }
@@ -373,13 +372,6 @@ inline unsigned blocks_of(int64_t n, int t) {
 }
 
 // ---------------------------------------------------------------- batched launches (persistent grids)
-__global__ void __launch_bounds__(256) k_batch_jacobi32(const BatchJacobi* __restrict__ a, const int* __restrict__ act,
-                                                        int N) {
-    batch_walk(a, act, N, [&](const BatchJacobi& A, VB vb) {
-        const MgLevel32 L = A.L;
-        jacobi_init32(vb, L, A.r, A.x, A.w, A.S);
-    });
-}
 __global__ void __launch_bounds__(256) k_batch_prolong_add32(const BatchProlongAdd* __restrict__ a,
                                                              const int* __restrict__ act, int N) {
     batch_walk(a, act, N, [&](const BatchProlongAdd& A, VB vb) {
@@ -402,12 +394,8 @@ constexpr int BATCH_GRID256 = 8 * 148, BATCH_GRID_LS = 148;
 
 }  // namespace
 
-int batch_blocks_jacobi(const BatchJacobi& a) { return (int)blocks_of(a.L.nn, 256); }
 int batch_blocks_prolong_add(const BatchProlongAdd& a) { return (int)blocks_of(a.Lf.nn, 256); }
 int batch_blocks_level_op(const BatchLevelOp& a) { return (int)blocks_of(a.L.nn, LS_NODES); }
-void launch_batch_jacobi32(const BatchJacobi* a, const int* act, int N, cudaStream_t s) {
-    k_batch_jacobi32<<<BATCH_GRID256, 256, 0, s>>>(a, act, N);
-}
 void launch_batch_prolong_add32(const BatchProlongAdd* a, const int* act, int N, cudaStream_t s) {
     k_batch_prolong_add32<<<BATCH_GRID256, 256, 0, s>>>(a, act, N);
 }

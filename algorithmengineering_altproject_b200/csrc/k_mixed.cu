@@ -492,9 +492,11 @@ __global__ void __launch_bounds__(COARSE_THREADS) k_coarse_solve32(MgLevel32 L, 
 
 // ---------------------------------------------------------------- PCG vector steps in FP32
 // r -= alpha Ap and |r|^2 (alpha = r.z / p.Ap of this iteration, stored for the direction kernel, which
-// applies x += alpha p while it reads p anyway)
+// applies x += alpha p while it reads p anyway).  With z, the Standard cycle's level-0 start z = w r / D (rd = 1/D) of
+// the new r too, which saves the pass that would read r again; fixed DOFs and pads have r = 0, so z = 0 there.
 __device__ __forceinline__ void pcg_update32(VB vb, int64_t NNp, float* __restrict__ r, const float* __restrict__ Ap,
-                                             RedSlot red, PcgScalars* S, double* sh) {
+                                             RedSlot red, PcgScalars* S, double* sh, const float* __restrict__ rd,
+                                             float* __restrict__ z, float w) {
     if (S->done) return;
     const double den = S->denom;
     // breakdown of the FP32 recurrence (p.Ap <= 0 or r.z <= 0, e.g. an indefinite preconditioner): stop this
@@ -512,7 +514,7 @@ __device__ __forceinline__ void pcg_update32(VB vb, int64_t NNp, float* __restri
     if (vb.b == 0 && threadIdx.x == 0) S->alpha = alpha;
     // the three component planes are contiguous: one flat vector of 3 NNp floats (pads stay zero), 16-byte
     // accesses (cudaMalloc bases are 256-byte aligned; NNp is a multiple of 4)
-    const int n3 = (int)(3 * NNp), n4 = n3 >> 2;
+    const int n4 = (int)(3 * NNp) >> 2;
     const int stride = vb.n * blockDim.x;
     float4* __restrict__ r4 = reinterpret_cast<float4*>(r);
     const float4* __restrict__ a4 = reinterpret_cast<const float4*>(Ap);
@@ -523,13 +525,13 @@ __device__ __forceinline__ void pcg_update32(VB vb, int64_t NNp, float* __restri
         rv.x = fmaf(-alpha, av.x, rv.x); rv.y = fmaf(-alpha, av.y, rv.y);
         rv.z = fmaf(-alpha, av.z, rv.z); rv.w = fmaf(-alpha, av.w, rv.w);
         r4[i] = rv;
+        if (z) {
+            const float4 dv = reinterpret_cast<const float4*>(rd)[i];
+            reinterpret_cast<float4*>(z)[i] =
+                make_float4((w * rv.x) * dv.x, (w * rv.y) * dv.y, (w * rv.z) * dv.z, (w * rv.w) * dv.w);
+        }
         part += (double)fmaf(rv.w, rv.w, fmaf(rv.z, rv.z, fmaf(rv.y, rv.y, rv.x * rv.x)));
-    }
-    for (int i = 4 * n4 + vb.b * blockDim.x + threadIdx.x; i < n3; i += stride) {
-        const float rv = fmaf(-alpha, Ap[i], r[i]);
-        r[i] = rv;
-        part = fma((double)rv, (double)rv, part);
-    }
+    }   // NNp is a multiple of 4: no remainder
     double tot;
     if (grid_fold(part, red, sh, &tot, vb) && threadIdx.x == 0) {
         S->rnorm2 = tot;
@@ -544,9 +546,10 @@ __device__ __forceinline__ void pcg_update32(VB vb, int64_t NNp, float* __restri
 }
 __global__ void __launch_bounds__(RED_THREADS) k_pcg_update32(Grid g, float* __restrict__ r,
                                                               const float* __restrict__ Ap, RedSlot red,
-                                                              PcgScalars* S) {
+                                                              PcgScalars* S, const float* __restrict__ rd,
+                                                              float* __restrict__ z, float w) {
     __shared__ double sh[32];
-    pcg_update32(vb_real(), g.NNp, r, Ap, red, S, sh);
+    pcg_update32(vb_real(), g.NNp, r, Ap, red, S, sh, rd, z, w);
 }
 
 // x += alpha p_old and, unless the update just converged, p = z + beta p_old.  Once converged, the
@@ -607,7 +610,7 @@ __global__ void k_batch_compact(const BatchCompact* __restrict__ jobs, int njobs
 __global__ void __launch_bounds__(RED_THREADS) k_batch_update32(const BatchUpdate* __restrict__ a,
                                                                 const int* __restrict__ act, int N) {
     __shared__ double sh[32];
-    batch_walk(a, act, N, [&](const BatchUpdate& A, VB vb) { pcg_update32(vb, A.NNp, A.r, A.Ap, A.red, A.S, sh); });
+    batch_walk(a, act, N, [&](const BatchUpdate& A, VB vb) { pcg_update32(vb, A.NNp, A.r, A.Ap, A.red, A.S, sh, A.rd, A.z, A.w); });
 }
 
 __global__ void __launch_bounds__(RED_THREADS) k_batch_direction32(const BatchDirection* __restrict__ a,
@@ -767,11 +770,9 @@ void launch_coarse_solve32(const MgLevel32& L, const double* X, int N, const int
     k_coarse_solve32<<<blocks, COARSE_THREADS, (size_t)((N > 0 ? N : 0) + 32 * COARSE_WARPS) * sizeof(double), s>>>(
         L, X, N, status, S);
 }
-void launch_pcg_update32(const Grid& g, float* x, float* r, const float* p, const float* Ap, RedSlot red,
-                         PcgScalars* S, cudaStream_t s) {
-    (void)x;
-    (void)p;
-    k_pcg_update32<<<update32_blocks(g.NNp), RED_THREADS, 0, s>>>(g, r, Ap, red, S);
+void launch_pcg_update32(const Grid& g, float* r, const float* Ap, RedSlot red, PcgScalars* S, const float* rd, float* z,
+                         float w, cudaStream_t s) {
+    k_pcg_update32<<<update32_blocks(g.NNp), RED_THREADS, 0, s>>>(g, r, Ap, red, S, rd, z, w);
 }
 void launch_pcg_direction32(const Grid& g, const float* z, float* p, float* x, PcgScalars* S, cudaStream_t s) {
     k_pcg_direction32<<<update32_blocks(g.NNp), RED_THREADS, 0, s>>>(g, z, p, x, S);

@@ -278,8 +278,9 @@ void launch_prolong_smooth0_32(const MgLevel32& Lc, const MgLevel32& Lf, const f
                                float w, RedSlot dot, PcgScalars* S, cudaStream_t s);
 void launch_coarse_solve32(const MgLevel32& L, const double* X, int N, const int* status, const PcgScalars* S,
                            cudaStream_t s);
-void launch_pcg_update32(const Grid& g, float* x, float* r, const float* p, const float* Ap, RedSlot red,
-                         PcgScalars* S, cudaStream_t s);
+// with z: the Standard cycle's level-0 start z = w r / D (rd = 1/D) of the new r too
+void launch_pcg_update32(const Grid& g, float* r, const float* Ap, RedSlot red, PcgScalars* S, const float* rd, float* z,
+                         float w, cudaStream_t s);
 // p = z + beta p and the deferred x += alpha p of the same iteration (see PcgScalars::xit)
 void launch_pcg_direction32(const Grid& g, const float* z, float* p, float* x, PcgScalars* S, cudaStream_t s);
 
@@ -335,12 +336,15 @@ struct BatchMatvec {      // K(E)u in the TMA tile shapes (maps in global memory
     const float* rd;      // mode 2: 1/D
     float omega;          // mode 2: Jacobi weight
 };
-struct BatchUpdate {      // r -= alpha Ap with |r|^2
+struct BatchUpdate {      // r -= alpha Ap with |r|^2; with z the Standard cycle's level-0 start z = w r / D too
     int64_t NNp;
     float* r;
     const float* Ap;
     RedSlot red;
     PcgScalars* S;
+    const float* rd;
+    float* z;
+    float w;
 };
 struct BatchDirection {   // x += alpha p, p = z + beta p
     int64_t NNp;
@@ -379,13 +383,6 @@ struct BatchCoarse {      // coarsest-level solve
     const int* status;
     PcgScalars* S;
 };
-struct BatchJacobi {      // the Standard cycle's finest-level start x = w r / D
-    MgLevel32 L;
-    const float* r;
-    float* x;
-    float w;
-    PcgScalars* S;
-};
 struct BatchProlongAdd {  // xo = xi + P xc
     MgLevel32 Lc, Lf;
     const float* xc;
@@ -402,10 +399,8 @@ struct BatchLevelOp {     // y = r - K_l x, or y = x + w (r - K_l x) / D, from t
     float w;
     PcgScalars* S;
 };
-int batch_blocks_jacobi(const BatchJacobi& a);
 int batch_blocks_prolong_add(const BatchProlongAdd& a);
 int batch_blocks_level_op(const BatchLevelOp& a);
-void launch_batch_jacobi32(const BatchJacobi* a, const int* act, int N, cudaStream_t s);
 void launch_batch_prolong_add32(const BatchProlongAdd* a, const int* act, int N, cudaStream_t s);
 void launch_batch_level_op32(const BatchLevelOp* a, const int* act, int N, bool correct, cudaStream_t s);
 
