@@ -673,7 +673,7 @@ static int vcycle_launches(const Context* c) {
     int n = 0;
     if (c->standard) {
         for (int l = 1; l < L; ++l) n += restrict_launches(c->lv[l]);
-        return n + 3 * (L - 2) + 8;
+        return n + 3 * (L - 2) + 6;
     }
     const int tail = adapted_tail_first(c->lv, L, c->Nc), down = std::min(tail, L - 1);
     for (int l = 1; l <= down; ++l) n += restrict_launches(c->lv[l]);
@@ -689,8 +689,7 @@ static void vcycle_standard(Context* c, const double* r, double* z, PcgScalars* 
     const double* Kd = c->ke_pat ? c->Kd : nullptr;
     c->launches += vcycle_launches(c);
     launch_jacobi_init(c->lv[0], r, z, w, S, c->st);
-    launch_matvec64_stream(c->g, c->st64, c->Ke_h, Kd, c->E_mg, c->mask0, z, c->Ap, S, c->st);
-    launch_residual(c->lv[0], r, c->Ap, S, c->st);
+    launch_residual64_stream(c->g, c->st64, c->Ke_h, Kd, c->E_mg, c->mask0, z, r, c->Ap, S, c->st);
     for (int l = 0; l + 1 < L; ++l) {
         const MgLevel &Lf = c->lv[l], &Lc = c->lv[l + 1];
         if (l > 0) launch_level_op(Lf, c->KelT[l], Lf.x, Lf.r, c->vtmp[l], false, w, S, c->st);
@@ -701,13 +700,12 @@ static void vcycle_standard(Context* c, const double* r, double* z, PcgScalars* 
     const double* xc = c->lv[L - 1].x;
     for (int l = L - 2; l >= 1; --l) {
         const MgLevel& Lf = c->lv[l];
-        launch_prolong_add(c->lv[l + 1], Lf, xc, Lf.x, S, c->st);
+        launch_prolong_add(c->lv[l + 1], Lf, xc, Lf.x, Lf.x, S, c->st);
         launch_level_op(Lf, c->KelT[l], Lf.x, Lf.r, c->vtmp[l], true, w, S, c->st);
         xc = c->vtmp[l];
     }
-    launch_prolong_add(c->lv[1], c->lv[0], xc, z, S, c->st);
-    launch_matvec64_stream(c->g, c->st64, c->Ke_h, Kd, c->E_mg, c->mask0, z, c->Ap, S, c->st);
-    launch_jacobi_correct(c->lv[0], r, c->Ap, z, w, S, c->st);
+    launch_prolong_add(c->lv[1], c->lv[0], xc, z, c->Ap, S, c->st);
+    launch_correct64_stream(c->g, c->st64, c->Ke_h, Kd, c->E_mg, c->mask0, c->Ap, r, c->lv[0].diag, w, z, S, c->st);
     if (S) launch_dot_rz(c->g.NN, r, z, dot, S, c->st);
 }
 

@@ -112,13 +112,17 @@ struct S64Loads {
 };
 static_assert(S64_BX == 32 && S64_BY >= 2 && S64::PY <= 32, "S64Loads: warps 0 and 1 take the last row and column");
 
-template <bool PAT>
+// MODE 0: y = K u;  1: the Standard V-cycle's residual y = r - K u;  2: its correction y = u + w (r - K u) / D, y other
+// than u.  Fixed DOFs 0.  As one pass each, modes 1 and 2 save the two that read K u again.
+template <bool PAT, int MODE>
 __global__ void __launch_bounds__(S64::NT, 2) k_matvec64_stream(Grid g, Stream64Tiling t, const Ke64 ke,
                                                                 const double* __restrict__ Kd,
                                                                 const double* __restrict__ E,
                                                                 const uint8_t* __restrict__ mask,
                                                                 const double* __restrict__ u,
-                                                                double* __restrict__ y, const PcgScalars* S) {
+                                                                double* __restrict__ y, const PcgScalars* S,
+                                                                const double* __restrict__ r,
+                                                                const double* __restrict__ diag, double w_jac) {
     extern __shared__ __align__(16) double sm[];
     if (S != nullptr && S->done) return;
     constexpr int BX = S64::BX, BY = S64::BY, NT = S64::NT, PX = S64::PX, AREA = S64::PY * S64::PX;
@@ -204,6 +208,19 @@ __global__ void __launch_bounds__(S64::NT, 2) k_matvec64_stream(Grid g, Stream64
             if (k >= 1 && tx < BX - 1 && ty < BY - 1) {
                 const int ix = X0 + tx, iy = Y0 + ty, iz = cz;
                 if (ix < g.nnx && iy < g.nny) {
+                    const int64_t n = g.node(ix, iy, iz);
+                    const int mk = mask[n];
+                    double r0 = 0.0, r1 = 0.0, r2 = 0.0, d0 = 1.0, d1 = 1.0, d2 = 1.0;
+                    if (MODE != 0) {
+                        r0 = r[n];
+                        r1 = r[NN + n];
+                        r2 = r[2 * NN + n];
+                    }
+                    if (MODE == 2) {
+                        d0 = diag[n];
+                        d1 = diag[NN + n];
+                        d2 = diag[2 * NN + n];
+                    }
                     const double* Ebelow = sm + S64::EMOD + ((k - 1) % 3) * NT;
                     const double* Eabove = sm + S64::EMOD + (k % 3) * NT;
                     const double* Fbelow = sm + S64::FT + ((k - 1) & 1) * 12 * NT;
@@ -230,8 +247,17 @@ __global__ void __launch_bounds__(S64::NT, 2) k_matvec64_stream(Grid g, Stream64
                             y2 = fma(F[2 * NT], Ec, y2);
                         }
                     }
-                    const int64_t n = g.node(ix, iy, iz);
-                    const int mk = mask[n];
+                    if (MODE != 0) {
+                        y0 = r0 - y0;
+                        y1 = r1 - y1;
+                        y2 = r2 - y2;
+                    }
+                    if (MODE == 2) {
+                        const double* U = sm + S64::PLANE + (k % 3) * S64::PLANE_SZ + (ty + 1) * PX + tx + 1;
+                        y0 = U[0] + (w_jac * y0) * (1.0 / (1.0e-30 < d0 ? d0 : 1.0e-30));
+                        y1 = U[AREA] + (w_jac * y1) * (1.0 / (1.0e-30 < d1 ? d1 : 1.0e-30));
+                        y2 = U[2 * AREA] + (w_jac * y2) * (1.0 / (1.0e-30 < d2 ? d2 : 1.0e-30));
+                    }
                     if (mk & 1) y0 = 0.0;
                     if (mk & 2) y1 = 0.0;
                     if (mk & 4) y2 = 0.0;
@@ -269,7 +295,8 @@ bool ke_pattern_magnitudes(const double* Ke, double* D) {
 
 int stream64_tiling(const Grid& g, int dev, Stream64Tiling* t) {
     int per_sm = 1 << 30, sms = 0;
-    for (auto fn : {k_matvec64_stream<true>, k_matvec64_stream<false>}) {
+    for (auto fn : {k_matvec64_stream<true, 0>, k_matvec64_stream<false, 0>, k_matvec64_stream<true, 1>,
+                    k_matvec64_stream<false, 1>, k_matvec64_stream<true, 2>, k_matvec64_stream<false, 2>}) {
         cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S64::BYTES);
         if (e != cudaSuccess) return set_cuda_error(e, "cudaFuncSetAttribute", __FILE__, __LINE__);
         int n = 0;
@@ -304,17 +331,36 @@ int stream64_tiling(const Grid& g, int dev, Stream64Tiling* t) {
     return T3D_OK;
 }
 
-void launch_matvec64_stream(const Grid& g, const Stream64Tiling& t, const double* Ke_host, const double* Kd,
-                            const double* E, const uint8_t* mask, const double* u, double* y, const PcgScalars* S,
-                            cudaStream_t s) {
+namespace {
+template <int MODE>
+void launch_stream(const Grid& g, const Stream64Tiling& t, const double* Ke_host, const double* Kd, const double* E,
+                   const uint8_t* mask, const double* u, double* y, const PcgScalars* S, const double* r,
+                   const double* diag, double w, cudaStream_t s) {
     if (Kd) {   // the by-value Ke is not read in this form
         static const Ke64 unused{};
-        k_matvec64_stream<true><<<t.grid, S64::NT, S64::BYTES, s>>>(g, t, unused, Kd, E, mask, u, y, S);
+        k_matvec64_stream<true, MODE><<<t.grid, S64::NT, S64::BYTES, s>>>(g, t, unused, Kd, E, mask, u, y, S, r, diag, w);
         return;
     }
     Ke64 ke;
     for (int i = 0; i < 576; ++i) ke.v[i] = Ke_host[i];
-    k_matvec64_stream<false><<<t.grid, S64::NT, S64::BYTES, s>>>(g, t, ke, nullptr, E, mask, u, y, S);
+    k_matvec64_stream<false, MODE><<<t.grid, S64::NT, S64::BYTES, s>>>(g, t, ke, nullptr, E, mask, u, y, S, r, diag, w);
+}
+}  // namespace
+
+void launch_matvec64_stream(const Grid& g, const Stream64Tiling& t, const double* Ke_host, const double* Kd,
+                            const double* E, const uint8_t* mask, const double* u, double* y, const PcgScalars* S,
+                            cudaStream_t s) {
+    launch_stream<0>(g, t, Ke_host, Kd, E, mask, u, y, S, nullptr, nullptr, 0.0, s);
+}
+void launch_residual64_stream(const Grid& g, const Stream64Tiling& t, const double* Ke_host, const double* Kd,
+                              const double* E, const uint8_t* mask, const double* u, const double* r, double* y,
+                              const PcgScalars* S, cudaStream_t s) {
+    launch_stream<1>(g, t, Ke_host, Kd, E, mask, u, y, S, r, nullptr, 0.0, s);
+}
+void launch_correct64_stream(const Grid& g, const Stream64Tiling& t, const double* Ke_host, const double* Kd,
+                             const double* E, const uint8_t* mask, const double* u, const double* r, const double* diag,
+                             double w, double* y, const PcgScalars* S, cudaStream_t s) {
+    launch_stream<2>(g, t, Ke_host, Kd, E, mask, u, y, S, r, diag, w, s);
 }
 
 void launch_dot_pcg(const Grid& g, const double* p, const double* Ap, RedSlot red, PcgScalars* S, cudaStream_t s) {

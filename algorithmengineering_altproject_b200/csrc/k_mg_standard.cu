@@ -309,33 +309,12 @@ __global__ void k_jacobi_init(MgLevel L, const double* __restrict__ r, double* _
         x[c * L.nn + n] = ((m >> c) & 1) ? 0.0 : (w * r[c * L.nn + n]) * inv_diag(L, c, n);
 }
 
-// d = r - Kx (in place on Kx)
-__global__ void k_residual(MgLevel L, const double* __restrict__ r, double* __restrict__ kx, const PcgScalars* S) {
+// xo = xi + P xc (trilinear from the coarse cell floor(f/s), clamped to the last cell), fixed DOFs 0; xo may be xi.
+// One thread per node and component (blockIdx.y).
+__global__ void __launch_bounds__(256) k_prolong_add(MgLevel Lc, MgLevel Lf, const double* __restrict__ xc,
+                                                     const double* xi, double* xo, const PcgScalars* S) {
     if (S != nullptr && S->done) return;
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= L.nn) return;
-    const int m = L.mask[n];
-    for (int c = 0; c < 3; ++c) kx[c * L.nn + n] = ((m >> c) & 1) ? 0.0 : r[c * L.nn + n] - kx[c * L.nn + n];
-}
-
-// x += w (r - Kx) / D
-__global__ void k_jacobi_correct(MgLevel L, const double* __restrict__ r, const double* __restrict__ kx,
-                                 double* __restrict__ x, double w, const PcgScalars* S) {
-    if (S != nullptr && S->done) return;
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= L.nn) return;
-    const int m = L.mask[n];
-    for (int c = 0; c < 3; ++c) {
-        const int64_t i = c * L.nn + n;
-        x[i] = ((m >> c) & 1) ? 0.0 : x[i] + (w * (r[i] - kx[i])) * inv_diag(L, c, n);
-    }
-}
-
-// xf += P xc (trilinear from the coarse cell floor(f/s), clamped to the last cell), fixed DOFs 0
-__global__ void k_prolong_add(MgLevel Lc, MgLevel Lf, const double* __restrict__ xc, double* __restrict__ xf,
-                              const PcgScalars* S) {
-    if (S != nullptr && S->done) return;
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+    const int n = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
     if (n >= Lf.nn) return;
     const int s = Lc.span;
     const int fnx = Lf.nx + 1, fny = Lf.ny + 1;
@@ -344,15 +323,14 @@ __global__ void k_prolong_add(MgLevel Lc, MgLevel Lf, const double* __restrict__
     if (cx >= Lc.nx) cx = Lc.nx - 1;
     if (cy >= Lc.ny) cy = Lc.ny - 1;
     if (cz >= Lc.nz) cz = Lc.nz - 1;
-    const int m = Lf.mask[n];
-    for (int c = 0; c < 3; ++c) {
-        double p = 0.0;
-        for (int A = 0; A < 8; ++A)
-            p = p + tri_w(s, fx - cx * s, fy - cy * s, fz - cz * s, A) *
-                        xc[c * Lc.nn + lnode(Lc, cx + corner_dx(A), cy + corner_dy(A), cz + corner_dz(A))];
-        const int64_t i = c * Lf.nn + n;
-        xf[i] = ((m >> c) & 1) ? 0.0 : xf[i] + p;
-    }
+    const double* __restrict__ X = xc + c * Lc.nn;
+    double p = 0.0;
+#pragma unroll
+    for (int A = 0; A < 8; ++A)
+        p = p + tri_w(s, fx - cx * s, fy - cy * s, fz - cz * s, A) *
+                    X[lnode(Lc, cx + corner_dx(A), cy + corner_dy(A), cz + corner_dz(A))];
+    const int64_t i = c * Lf.nn + n;
+    xo[i] = ((Lf.mask[n] >> c) & 1) ? 0.0 : xi[i] + p;
 }
 
 // r.z in the canonical order; the last block sets rz (first use) or beta = rz_new/max(1e-30,rz), rz = rz_new
@@ -472,16 +450,9 @@ void launch_level_op(const MgLevel& L, const double* Kel, const double* x, const
 void launch_jacobi_init(const MgLevel& L, const double* r, double* x, double w, const PcgScalars* S, cudaStream_t s) {
     k_jacobi_init<<<blocks_of(L.nn, 256), 256, 0, s>>>(L, r, x, w, S);
 }
-void launch_residual(const MgLevel& L, const double* r, double* kx, const PcgScalars* S, cudaStream_t s) {
-    k_residual<<<blocks_of(L.nn, 256), 256, 0, s>>>(L, r, kx, S);
-}
-void launch_jacobi_correct(const MgLevel& L, const double* r, const double* kx, double* x, double w,
-                           const PcgScalars* S, cudaStream_t s) {
-    k_jacobi_correct<<<blocks_of(L.nn, 256), 256, 0, s>>>(L, r, kx, x, w, S);
-}
-void launch_prolong_add(const MgLevel& Lc, const MgLevel& Lf, const double* xc, double* xf, const PcgScalars* S,
-                        cudaStream_t s) {
-    k_prolong_add<<<blocks_of(Lf.nn, 256), 256, 0, s>>>(Lc, Lf, xc, xf, S);
+void launch_prolong_add(const MgLevel& Lc, const MgLevel& Lf, const double* xc, const double* xi, double* xo,
+                        const PcgScalars* S, cudaStream_t s) {
+    k_prolong_add<<<dim3(blocks_of(Lf.nn, 256), 3), 256, 0, s>>>(Lc, Lf, xc, xi, xo, S);
 }
 void launch_dot_rz(int64_t NN, const double* r, const double* z, RedSlot red, PcgScalars* S, cudaStream_t s) {
     k_dot_rz<<<red_blocks(NN), RED_THREADS, 0, s>>>(NN, r, z, red, S);

@@ -92,6 +92,13 @@ void launch_matvec64_stream(const Grid& g, const Stream64Tiling& t, const double
                             const double* E, const uint8_t* mask, const double* u, double* y, const PcgScalars* S,
                             cudaStream_t s);
 // S->denom = p.Ap (3 components) in the canonical reduction order, unless S->done
+// the same with the Standard V-cycle's step: y = r - K u, and y = u + w (r - K u) / D (y other than u)
+void launch_residual64_stream(const Grid& g, const Stream64Tiling& t, const double* Ke_host, const double* Kd,
+                              const double* E, const uint8_t* mask, const double* u, const double* r, double* y,
+                              const PcgScalars* S, cudaStream_t s);
+void launch_correct64_stream(const Grid& g, const Stream64Tiling& t, const double* Ke_host, const double* Kd,
+                             const double* E, const uint8_t* mask, const double* u, const double* r, const double* diag,
+                             double w, double* y, const PcgScalars* S, cudaStream_t s);
 void launch_dot_pcg(const Grid& g, const double* p, const double* Ap, RedSlot red, PcgScalars* S, cudaStream_t s);
 void launch_compliance64(const Grid& g, const double* Ke, const double* E, const double* u, double* ce,
                          RedSlot red, double* C, cudaStream_t s);
@@ -159,11 +166,9 @@ void launch_level_diag(const MgLevel& L, const double* Kel, cudaStream_t s);
 void launch_level_op(const MgLevel& L, const double* KelT, const double* x, const double* r, double* y, bool correct,
                      double w, const PcgScalars* S, cudaStream_t s);
 void launch_jacobi_init(const MgLevel& L, const double* r, double* x, double w, const PcgScalars* S, cudaStream_t s);
-void launch_residual(const MgLevel& L, const double* r, double* kx, const PcgScalars* S, cudaStream_t s);
-void launch_jacobi_correct(const MgLevel& L, const double* r, const double* kx, double* x, double w,
-                           const PcgScalars* S, cudaStream_t s);
-void launch_prolong_add(const MgLevel& Lc, const MgLevel& Lf, const double* xc, double* xf, const PcgScalars* S,
-                        cudaStream_t s);
+// xo = xi + P xc, fixed DOFs 0; xo may be xi
+void launch_prolong_add(const MgLevel& Lc, const MgLevel& Lf, const double* xc, const double* xi, double* xo,
+                        const PcgScalars* S, cudaStream_t s);
 void launch_dot_rz(int64_t NN, const double* r, const double* z, RedSlot red, PcgScalars* S, cudaStream_t s);
 void launch_to_coarse_layout(const MgLevel& L, const double* Kel, double* Kce, cudaStream_t s);
 
