@@ -69,16 +69,18 @@ __global__ void k_mask_restrict(MgLevel Lc, MgLevel Lf) {
 // ------------------------------------------------------------------ coarse diagonal (diagonal.cpp:66-138)
 // Gather per coarse DOF: incident coarse elements in colour order, their (s+1)^3 sub-nodes in
 // (iz,iy,ix) order, weight W_a^2, skipping fixed coarse or fine DOFs.
-__global__ void k_diag_coarsen(MgLevel Lc, MgLevel Lf) {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+// One thread per node and component (blockIdx.y).  The order is a chain of 8 (s+1)^3 additions; a row of sub-nodes is
+// loaded ahead of it, and a skipped sub-node (fixed, or in no element) adds +0, which changes no sum.
+__global__ void __launch_bounds__(64) k_diag_coarsen(MgLevel Lc, MgLevel Lf) {
+    const int n = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
     if (n >= Lc.nn) return;
     const LevelIdx C(Lc), F(Lf);
     const int X = n % C.nnx, Y = (n / C.nnx) % C.nny, Z = n / (C.nnx * C.nny);
     const int s = Lc.span;
-    const int cm = Lc.mask[n];
-    const int64_t fNN = Lf.nn;
-    double dc[3] = {0, 0, 0}, ws[3] = {0, 0, 0};
-    for (int col = 0; col < 8; ++col) {
+    const bool fixed = (Lc.mask[n] >> c) & 1;
+    const double* __restrict__ fd = Lf.diag + c * Lf.nn;
+    double dc = 0.0, ws = 0.0;
+    for (int col = 0; col < 8 && !fixed; ++col) {
         const int ccx = (((X - 1) & 1) == (col & 1)) ? X - 1 : X;
         const int ccy = (((Lc.ny - Y) & 1) == ((col >> 1) & 1)) ? Y - 1 : Y;
         const int ccz = (((Z - 1) & 1) == ((col >> 2) & 1)) ? Z - 1 : Z;
@@ -86,28 +88,31 @@ __global__ void k_diag_coarsen(MgLevel Lc, MgLevel Lf) {
         const int a = corner_of(X - ccx, Y - ccy, Z - ccz);
         const int fx0 = ccx * s, fy0 = (ccy + 1) * s, fz0 = ccz * s;
         for (int iz = 0; iz <= s; ++iz)
-            for (int iy = 0; iy <= s; ++iy)
-                for (int ix = 0; ix <= s; ++ix) {
+#pragma unroll 5
+            for (int iy = 0; iy <= s; ++iy) {
+                double d[5];
+                bool on[5];
+#pragma unroll
+                for (int ix = 0; ix < 5; ++ix) {
                     const int fn = F.node(fx0 + ix, fy0 - iy, fz0 + iz);
-                    const double w = corner_weight(s, ix, iy, iz, a);
-                    const double w2 = w * w;
-                    const int fm = Lf.mask[fn];
-                    for (int c = 0; c < 3; ++c) {
-                        if (((cm >> c) & 1) || ((fm >> c) & 1)) continue;
-                        dc[c] = dc[c] + w2 * Lf.diag[c * fNN + fn];
-                        ws[c] = ws[c] + w2;
-                    }
+                    on[ix] = ix <= s && !((Lf.mask[ix <= s ? fn : 0] >> c) & 1);
+                    d[ix] = ix <= s ? fd[fn] : 0.0;
                 }
+#pragma unroll
+                for (int ix = 0; ix < 5; ++ix) {
+                    const double w = corner_weight(s, ix, iy, iz, a);
+                    const double w2 = on[ix] ? w * w : 0.0;
+                    dc = dc + w2 * (on[ix] ? d[ix] : 0.0);
+                    ws = ws + w2;
+                }
+            }
     }
-    for (int c = 0; c < 3; ++c) {
-        double v;
-        if ((cm >> c) & 1) v = 1.0;
-        else if (ws[c] > 0) {
-            v = dc[c] / ws[c];
-            if (!(v > 0.0)) v = 1.0;
-        } else v = 1.0;
-        Lc.diag[c * Lc.nn + n] = v;
+    double v = 1.0;
+    if (!fixed && ws > 0) {
+        v = dc / ws;
+        if (!(v > 0.0)) v = 1.0;
     }
+    Lc.diag[c * Lc.nn + n] = v;
 }
 
 // ------------------------------------------------------------------ restriction (transfers.cpp:449-533)
@@ -188,20 +193,18 @@ __global__ void __launch_bounds__(128) k_restrict_yz(MgLevel Lc, MgLevel Lf, con
     const int cnx = Lc.nx + 1, cny = Lc.ny + 1, fny = Lf.ny + 1, fnz = Lf.nz + 1;
     const int cx = n % cnx, cy = (n / cnx) % cny, cz = n / (cnx * cny);
     const double* __restrict__ a = a1 + c * ((int64_t)fnz * fny * cnx) + cx;
+    double q[WS * WS];   // the whole window in flight; points outside the grid load nothing and add +0 (no change)
+#pragma unroll
+    for (int k = 0; k < WS * WS; ++k) {
+        const int fy = cy * SP + k % WS - (SP - 1), fz = cz * SP + k / WS - (SP - 1);
+        q[k] = fz >= 0 && fz < fnz && fy >= 0 && fy < fny ? a[(fz * fny + fy) * cnx] : 0.0;
+    }
     double v = 0.0;
 #pragma unroll
     for (int iz = 0; iz < WS; ++iz) {
-        const int fz = cz * SP + iz - (SP - 1);
-        const bool zin = fz >= 0 && fz < fnz;
-        double q[WS];
-#pragma unroll
-        for (int iy = 0; iy < WS; ++iy) {   // points outside the grid load nothing and add +0, which changes no sum
-            const int fy = cy * SP + iy - (SP - 1);
-            q[iy] = zin && fy >= 0 && fy < fny ? a[(fz * fny + fy) * cnx] : 0.0;
-        }
         double t = 0.0;
 #pragma unroll
-        for (int iy = 0; iy < WS; ++iy) t = t + hat(iy, SP) * q[iy];
+        for (int iy = 0; iy < WS; ++iy) t = t + hat(iy, SP) * q[iz * WS + iy];
         v = v + hat(iz, SP) * t;
     }
     restrict_store(Lc, n, c, restrict_scale(Lc, Lf, n, cx, cy, cz, c, v, normalize), rc, x0, w0);
@@ -682,7 +685,7 @@ void launch_mask_restrict(const MgLevel& Lc, const MgLevel& Lf, cudaStream_t s) 
     k_mask_restrict<<<blocks_for(Lc.nn, 128), 128, 0, s>>>(Lc, Lf);
 }
 void launch_diag_coarsen(const MgLevel& Lc, const MgLevel& Lf, cudaStream_t s) {
-    k_diag_coarsen<<<blocks_for(Lc.nn, 128), 128, 0, s>>>(Lc, Lf);
+    k_diag_coarsen<<<dim3(blocks_for(Lc.nn, 64), 3), 64, 0, s>>>(Lc, Lf);
 }
 // span 4 (the first transition): x pass, then the y-z pass; span 2: the whole window.  A separate y pass reads
 // less, and its two launches cost more up to about 10^5 coarse nodes.

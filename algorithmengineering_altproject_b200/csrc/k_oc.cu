@@ -209,13 +209,14 @@ __global__ void __launch_bounds__(256) k_oc_vec8(int64_t ne, const float* __rest
         }
         const int top = v8_top_binade(g0);
         const float inv_u = __int_as_float((127 + 23 - (top - V8_CAND + 1)) << 23);   // 1/u of the lowest binade
+#pragma unroll 2
         for (int b = 0; b < V8_CHUNK; ++b) {
-            float f = v[lane * V8_PAD + 8 * b + j] * inv_u;
+            const float f = v[lane * V8_PAD + 8 * b + j] * inv_u;
 #pragma unroll
-            for (int k = 0; k < V8_CAND; ++k) {
-                even[k] = even[k] + f;
-                odd[k] = odd[k] + f;
-                f = f * 0.5f;
+            for (int k = 0; k < V8_CAND; ++k) {   // f 2^-k, exact, each from f: no chain from binade to binade
+                const float fk = f * __int_as_float((127 - k) << 23);
+                even[k] = even[k] + fk;
+                odd[k] = odd[k] + fk;
             }
         }
         uint2* out = tab + ((g0 * 8 + j) * V8_CAND) * V8_CHUNKS + lane;
