@@ -517,39 +517,80 @@ __global__ void k_chol_rows(const double* __restrict__ LT, double* __restrict__ 
 // every row below takes its term L_ik x_k, so each row's running value receives its terms in increasing k
 // (forward) and decreasing i (backward) and is divided last -- the order of the row-oriented sums, bit for bit.
 // Rows above j are skipped in the forward pass: their values stay +0 and leave the others unchanged (each
-// running value there is +0 or 1, never -0).  The warp's lanes split the rows; the factor is read by columns
-// (LT) in the forward pass and by rows (Lrow) in the backward one, both coalesced.
-constexpr int INV_WARPS = 8;   // columns per block
+// running value there is +0 or 1, never -0).  The warp's lanes split the rows, NV = N/32 (rounded up) running values
+// in each lane's registers; the factor is read by columns (LT) in the forward pass and by rows (Lrow) in the backward
+// one, both coalesced and a step ahead of their use.  What bounds it is the chain of divisions, one per step; with the
+// running values in shared memory and the factor's loads in the chain it took 0.20, 0.53 and 1.39 ms for 135, 336 and
+// 675 unknowns, now 0.12, 0.22 and 0.51.
+constexpr int INV_WARPS = 4;   // columns per block
 constexpr int INV_MAX_N = 1000;   // the largest dense coarsest system (NlimitDofs)
+template <int NV>
 __global__ void __launch_bounds__(INV_WARPS * 32) k_coarse_inverse(const double* __restrict__ LT,
                                                                    const double* __restrict__ Lrow, int N,
                                                                    const int* __restrict__ status,
                                                                    double* __restrict__ X) {
-    extern __shared__ double xs_all[];   // [INV_WARPS][N]
     if (*status != 1) return;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int j = blockIdx.x * INV_WARPS + w;
     if (j >= N) return;   // the whole warp (no block barrier below)
-    double* xs = xs_all + (int64_t)w * N;
-    for (int i = lane; i < N; i += 32) xs[i] = (i == j) ? 1.0 : 0.0;
-    __syncwarp();
-    for (int k = j; k < N; ++k) {
-        const double xk = xs[k] / Lrow[(int64_t)k * N + k];
-        __syncwarp();
-        if (lane == (k & 31)) xs[k] = xk;
-        const double* __restrict__ Lk = LT + (int64_t)k * N;   // column k: L_ik at Lk[i]
-        for (int i = k + 1 + lane; i < N; i += 32) xs[i] = xs[i] - Lk[i] * xk;
-        __syncwarp();
+    double x[NV], a[NV], d;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) x[v] = v * 32 + lane == j ? 1.0 : 0.0;
+    // factor entries of step k's rows below (forward) or above (backward) it; others 0, which changes no value
+    auto below = [&](int k) {
+        d = k < N ? LT[(int64_t)k * N + k] : 1.0;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const int i = v * 32 + lane;
+            a[v] = k < N && i > k && i < N ? LT[(int64_t)k * N + i] : 0.0;
+        }
+    };
+    auto above = [&](int i) {
+        d = i >= 0 ? Lrow[(int64_t)i * N + i] : 1.0;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const int k = v * 32 + lane;
+            a[v] = k < i ? Lrow[(int64_t)i * N + k] : 0.0;
+        }
+    };
+    below(j);
+#pragma unroll
+    for (int vb = 0; vb < NV; ++vb) {
+        if (vb * 32 + 31 < j) continue;
+        for (int kk = 0; kk < 32; ++kk) {
+            const int k = vb * 32 + kk;
+            if (k < j || k >= N) continue;
+            const double xk = __shfl_sync(0xffffffffu, x[vb], kk) / d;
+            double q[NV];
+#pragma unroll
+            for (int v = vb; v < NV; ++v) q[v] = a[v] * xk;
+            below(k + 1);
+            if (lane == kk) x[vb] = xk;
+#pragma unroll
+            for (int v = vb; v < NV; ++v)
+                if (v * 32 + lane > k) x[v] = x[v] - q[v];
+        }
     }
-    for (int i = N - 1; i >= 0; --i) {
-        const double* __restrict__ Li = Lrow + (int64_t)i * N;
-        const double xi = xs[i] / Li[i];
-        __syncwarp();
-        if (lane == (i & 31)) xs[i] = xi;
-        for (int k = lane; k < i; k += 32) xs[k] = xs[k] - Li[k] * xi;
-        __syncwarp();
+    above(N - 1);
+#pragma unroll
+    for (int vb = NV - 1; vb >= 0; --vb) {
+        for (int kk = 31; kk >= 0; --kk) {
+            const int i = vb * 32 + kk;
+            if (i >= N) continue;
+            const double xi = __shfl_sync(0xffffffffu, x[vb], kk) / d;
+            double q[NV];
+#pragma unroll
+            for (int v = 0; v <= vb; ++v) q[v] = a[v] * xi;
+            above(i - 1);
+            if (lane == kk) x[vb] = xi;
+#pragma unroll
+            for (int v = 0; v <= vb; ++v)
+                if (v * 32 + lane < i) x[v] = x[v] - q[v];
+        }
     }
-    for (int i = lane; i < N; i += 32) X[(int64_t)j * N + i] = xs[i];
+#pragma unroll
+    for (int v = 0; v < NV; ++v)
+        if (v * 32 + lane < N) X[(int64_t)j * N + v * 32 + lane] = x[v];
 }
 
 // Coarsest solve x_i = sum_j X[i][j] r_j (sequential in j) when the factorisation succeeded, else
@@ -740,12 +781,11 @@ int launch_cholesky(const double* A, double* LT, double* Lrow, int N, int* statu
 }
 void launch_coarse_inverse(const double* LT, const double* Lrow, int N, const int* status, double* X,
                            cudaStream_t s) {
-    const size_t smem = (size_t)N * INV_WARPS * sizeof(double);   // N <= 1000: at most 64 KB
-    // the attribute is per function, not per launch: always the bound for the largest N, so that contexts set
-    // up concurrently from several host threads never lower it under another thread's launch
-    cudaFuncSetAttribute(k_coarse_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(INV_MAX_N * INV_WARPS * sizeof(double)));
-    k_coarse_inverse<<<blocks_for(N, INV_WARPS), INV_WARPS * 32, smem, s>>>(LT, Lrow, N, status, X);
+    const unsigned b = blocks_for(N, INV_WARPS);
+    if (N <= 160) k_coarse_inverse<5><<<b, INV_WARPS * 32, 0, s>>>(LT, Lrow, N, status, X);
+    else if (N <= 352) k_coarse_inverse<11><<<b, INV_WARPS * 32, 0, s>>>(LT, Lrow, N, status, X);
+    else if (N <= 704) k_coarse_inverse<22><<<b, INV_WARPS * 32, 0, s>>>(LT, Lrow, N, status, X);
+    else k_coarse_inverse<32><<<b, INV_WARPS * 32, 0, s>>>(LT, Lrow, N, status, X);
 }
 void launch_coarse_solve(const MgLevel& L, const double* X, int N, const int* status, const PcgScalars* S,
                          cudaStream_t s) {
