@@ -35,12 +35,14 @@ __device__ __forceinline__ int lnode(const MgLevel& L, int x, int y, int z) {
     return (z * (L.ny + 1) + y) * (L.nx + 1) + x;
 }
 
-// level-1 element matrices from the finest grid: one CTA (576 threads, thread = entry (P, Q)) per GB
+// level-1 element matrices from the finest grid: one CTA (GT threads, thread = entries (P, Q) and (P + 12, Q)) per GB
 // consecutive coarse elements (cz*ny1 + cy)*nx1 + cx, so that each G_pos entry is read once per batch;
-// children are summed in position order, masked ones by the explicit product
-constexpr int GB = 16;
+// children are summed in position order, masked ones by the explicit product.  Two entries a thread: a pair of moduli
+// read from shared memory feeds 8 FP64 operations instead of 4, which was the bound with one, and two CTAs fit an SM
+// (256x512x256: 7.4 -> 5.9 ms; with one CTA and no spills 8.7).
+constexpr int GB = 16, GT = 288;
 
-__global__ void __launch_bounds__(576, 1) k_galerkin_fine(Grid g, MgLevel L1, int s, const double* __restrict__ E,
+__global__ void __launch_bounds__(GT, 2) k_galerkin_fine(Grid g, MgLevel L1, int s, const double* __restrict__ E,
                                                        const uint8_t* __restrict__ mask0,
                                                        const double* __restrict__ Gpos,
                                                        const double* __restrict__ Keg, double* __restrict__ Kel) {
@@ -69,7 +71,7 @@ __global__ void __launch_bounds__(576, 1) k_galerkin_fine(Grid g, MgLevel L1, in
         const int o = t / 8;
         wt[o][t % 8] = tri_w(s, o % s1, (o / s1) % s1, o / (s1 * s1), t % 8);
     }
-    kg[threadIdx.x] = Keg[threadIdx.x];
+    for (int t = threadIdx.x; t < 576; t += GT) kg[t] = Keg[t];
     __syncthreads();
     for (int q = threadIdx.x; q < GB * ns; q += blockDim.x) {
         const int b = q / ns, p = q % ns, ce = e0 + b;
@@ -103,65 +105,83 @@ __global__ void __launch_bounds__(576, 1) k_galerkin_fine(Grid g, MgLevel L1, in
     __syncthreads();
     const int P = threadIdx.x / 24, Q = threadIdx.x % 24;
     const int A = P / 3, r = P % 3, B = Q / 3, q = Q % 3;
-    const double* __restrict__ gcol = Gpos + threadIdx.x;
-    double acc[GB];
+    const double* __restrict__ gcol = Gpos + threadIdx.x;   // the second entry GT = 12 rows further: corner A + 4
+    double acc[2][GB];
 #pragma unroll
-    for (int b = 0; b < GB; ++b) acc[b] = 0.0;
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int b = 0; b < GB; ++b) acc[h][b] = 0.0;
     if (!masked) {
         // Every child is plain: acc_b += E_bp G_p[t] for all b in position order.  A skipped child (E_bp = 0)
         // adds +-0, which leaves acc unchanged (acc starts at +0 and a sum never turns into -0), so the sums are
-        // those of the per-child test below.  The next four children's G_pos entries load while four are summed.
-        double gn[4];
+        // those of the per-child test below.  The next two children's G_pos entries load while two are summed.
+        double gn[2][2];
 #pragma unroll
-        for (int v = 0; v < 4; ++v) gn[v] = gcol[v * 576];   // ns = s^3 is 8 or 64
-        for (int p0 = 0; p0 < ns; p0 += 4) {
-            double gc[4];
+        for (int v = 0; v < 2; ++v)
 #pragma unroll
-            for (int v = 0; v < 4; ++v) gc[v] = gn[v];
-            if (p0 + 4 < ns) {
+            for (int h = 0; h < 2; ++h) gn[v][h] = gcol[v * 576 + h * GT];   // ns = s^3 is 8 or 64
+#pragma unroll 1
+        for (int p0 = 0; p0 < ns; p0 += 2) {
+            double gc[2][2];
 #pragma unroll
-                for (int v = 0; v < 4; ++v) gn[v] = gcol[(p0 + 4 + v) * 576];
-            }
+            for (int v = 0; v < 2; ++v)
 #pragma unroll
-            for (int v = 0; v < 4; ++v) {
+                for (int h = 0; h < 2; ++h) {
+                    gc[v][h] = gn[v][h];
+                    if (p0 + 2 < ns) gn[v][h] = gcol[(p0 + 2 + v) * 576 + h * GT];
+                }
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
                 const double2* e2 = reinterpret_cast<const double2*>(&Ec[p0 + v][0]);
 #pragma unroll
-                for (int h = 0; h < GB / 2; ++h) {
-                    const double2 e = e2[h];
-                    acc[2 * h] = acc[2 * h] + e.x * gc[v];
-                    acc[2 * h + 1] = acc[2 * h + 1] + e.y * gc[v];
+                for (int i = 0; i < GB / 2; ++i) {
+                    const double2 e = e2[i];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        acc[h][2 * i] = acc[h][2 * i] + e.x * gc[v][h];
+                        acc[h][2 * i + 1] = acc[h][2 * i + 1] + e.y * gc[v][h];
+                    }
                 }
             }
         }
     } else {
+#pragma unroll 1
         for (int p = 0; p < ns; ++p) {
-            const double gp = gcol[p * 576];
+            const double gp[2] = {gcol[p * 576], gcol[p * 576 + GT]};
             const int i = p % s, j = (p / s) % s, k = p / (s * s);
 #pragma unroll
             for (int b = 0; b < GB; ++b) {
                 const double Ee = Ec[p][b];
                 if (Ee == 0.0) continue;
                 if (!anym[b][p]) {
-                    acc[b] = acc[b] + Ee * gp;
+                    acc[0][b] = acc[0][b] + Ee * gp[0];
+                    acc[1][b] = acc[1][b] + Ee * gp[1];
                 } else {   // sum_{a,c} w_aA w_cB M_ar M_cq E Ke[3a+r][3c+q]
                     // the inner sums u(a; r, B, q) = sum_c w_cB M_cq Ke[3a+r][3c+q] do not depend on A: thread
-                    // (3a+r, Q) forms its own once into us, and the outer sum over a reads them (the same terms in
-                    // the same order as summing u inside the loop over a).  The branch is the same for the block.
-                    double u = 0.0;
+                    // (3a+r, Q) forms its own two once into us, and the outer sum over a reads them (the same terms
+                    // in the same order as summing u inside the loop over a).  The branch is the same for the block.
+                    double u[2] = {0.0, 0.0};
+#pragma unroll 1
                     for (int c = 0; c < 8; ++c) {
                         if ((cmk[b][p][c] >> q) & 1) continue;
                         const double wc = wt[((k + corner_dz(c)) * s1 + j + corner_dy(c)) * s1 + i + corner_dx(c)][B];
-                        u = u + wc * kg[(3 * A + r) * 24 + 3 * c + q];
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) u[h] = u[h] + wc * kg[(3 * (A + 4 * h) + r) * 24 + 3 * c + q];
                     }
-                    us[threadIdx.x] = u;
+                    us[threadIdx.x] = u[0];
+                    us[threadIdx.x + GT] = u[1];
                     __syncthreads();
-                    double t = 0.0;
+                    double t[2] = {0.0, 0.0};
+#pragma unroll 1
                     for (int a = 0; a < 8; ++a) {
                         if ((cmk[b][p][a] >> r) & 1) continue;
-                        const double wa = wt[((k + corner_dz(a)) * s1 + j + corner_dy(a)) * s1 + i + corner_dx(a)][A];
-                        t = t + wa * us[(3 * a + r) * 24 + Q];
+                        const double* wa = wt[((k + corner_dz(a)) * s1 + j + corner_dy(a)) * s1 + i + corner_dx(a)];
+                        const double ua = us[(3 * a + r) * 24 + Q];
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) t[h] = t[h] + wa[A + 4 * h] * ua;
                     }
-                    acc[b] = acc[b] + Ee * t;
+                    acc[0][b] = acc[0][b] + Ee * t[0];
+                    acc[1][b] = acc[1][b] + Ee * t[1];
                     __syncthreads();   // us is rewritten by the next masked child
                 }
             }
@@ -171,9 +191,12 @@ __global__ void __launch_bounds__(576, 1) k_galerkin_fine(Grid g, MgLevel L1, in
     for (int b = 0; b < GB; ++b) {
         const int ce = e0 + b;
         if (ce >= ne1) continue;
-        double v = acc[b];
-        if (((cmask[b][A] >> r) & 1) || ((cmask[b][B] >> q) & 1)) v = 0.0;
-        Kel[(int64_t)ce * 576 + threadIdx.x] = v;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            double v = acc[h][b];
+            if (((cmask[b][A + 4 * h] >> r) & 1) || ((cmask[b][B] >> q) & 1)) v = 0.0;
+            Kel[(int64_t)ce * 576 + threadIdx.x + h * GT] = v;
+        }
     }
 }
 
@@ -426,7 +449,7 @@ void galerkin_positions(int s, const double* Ke, double* G) {
 
 void launch_galerkin_fine(const Grid& g, const MgLevel& L1, const double* E, const uint8_t* mask0, const double* Gpos,
                           const double* Ke, double* Kel, cudaStream_t s) {
-    k_galerkin_fine<<<blocks_of((int64_t)L1.nx * L1.ny * L1.nz, GB), 576, 0, s>>>(g, L1, L1.span, E, mask0, Gpos, Ke,
+    k_galerkin_fine<<<blocks_of((int64_t)L1.nx * L1.ny * L1.nz, GB), GT, 0, s>>>(g, L1, L1.span, E, mask0, Gpos, Ke,
                                                                               Kel);
 }
 void launch_galerkin_coarse(const MgLevel& Lf, const MgLevel& Lc, const double* Kf, double* Kc, cudaStream_t s) {
