@@ -139,8 +139,7 @@ class DesignServer:
         self._closed = False
         self._threads = []
         self._create_lock = threading.Lock()   # context creation (allocations, tile autotuning) one at a time
-        # first solves one at a time: run concurrently they occasionally gave one context a zero solid-domain
-        # compliance (cause not found); their design iterations still overlap
+        # first solves one at a time (each captures its PCG graph and fills the device); design iterations overlap
         self._init_lock = threading.Lock()
         self._warm = False
         self._joining = []          # batched engine: initialised requests waiting to join the batch
