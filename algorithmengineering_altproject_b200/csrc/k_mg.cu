@@ -685,6 +685,7 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) k_adapted_tail(TailLevels T, 
     if (*status != 1) {
         for (int i = threadIdx.x; i < 3 * nL; i += TAIL_THREADS)
             x[i] = coarse_jacobi(r[off + i], LL.diag[i], (LL.mask[i % nL] >> (i / nL)) & 1);
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");   // no copy of the inverse outlives the block
     } else {
         double* rs = x + 3 * nL;
         for (int j = threadIdx.x; j < N; j += TAIL_THREADS) rs[j] = r[off + (j % 3) * nL + j / 3];
