@@ -69,7 +69,7 @@ struct Batch {
     std::vector<void*> dallocs;
     bool standard = false;       // the members' V-cycle (all the same): Standard, else Adapted
     LaunchList mv, up, dir, p0, co, mv1, mv2;
-    LaunchList rs0[8], rs1[8], pr[8], lop[8], pa[8];
+    LaunchList rs0[8], rs1[8], pr[8], lsp[8], lnd[8], pa[8];   // level products: split levels, levels by nodes
     int maxL = 0, coarse_max = 0;
     CUtensorMap* maps = nullptr;
     std::vector<BatchCompact> compact;   // one compaction job per launch list
@@ -125,7 +125,7 @@ struct Batch {
         dflags = nullptr;
         err = nullptr;
         mv = up = dir = p0 = co = mv1 = mv2 = LaunchList{};
-        for (int l = 0; l < 8; ++l) rs0[l] = rs1[l] = pr[l] = lop[l] = pa[l] = LaunchList{};
+        for (int l = 0; l < 8; ++l) rs0[l] = rs1[l] = pr[l] = lsp[l] = lnd[l] = pa[l] = LaunchList{};
     }
 
     ~Batch() {
@@ -293,13 +293,18 @@ static int batch_lists(Batch* B) {
                           : BatchProlongAdd{Lc, Lf, xc, Lf.x, Lf.x, c->S32};
         }, [](const BatchProlongAdd& a) { return batch_blocks_prolong_add(a); }));
         if (l >= 1) {
-            CHECK(list(&B->lop[l], below, [l](t3d_context* c, int) {
+            auto op = [l](t3d_context* c, int) {
                 const MgLevel32& L = c->lv32[l];
                 return BatchLevelOp{L, c->Kel32[l], L.x, L.r, c->vtmp32[l], c->prm.mg_standard_weight, c->S32};
-            }, [](const BatchLevelOp& a) { return batch_blocks_level_op(a); }));
-            // each level product runs twice per cycle (down and up)
-            B->iter_kernels += 1;
-            B->iter_blocks += B->lop[l].blocks;
+            };
+            for (const bool split : {true, false}) {
+                LaunchList* L = split ? &B->lsp[l] : &B->lnd[l];
+                CHECK(list(L, [&](t3d_context* c) { return below(c) && batch_level_split(op(c, 0)) == split; }, op,
+                           [](const BatchLevelOp& a) { return batch_blocks_level_op(a); }));
+                // each level product runs twice per cycle (down and up)
+                B->iter_kernels += L->n > 0;
+                B->iter_blocks += L->blocks;
+            }
         }
     }
     if (B->standard) {
@@ -392,6 +397,13 @@ static void batch_restrict(Batch* B, int l) {
     if (B->rs1[l].n) launch_batch_restrict32(args_of<BatchRestrict>(B->rs1[l]), B->rs1[l].act, B->rs1[l].n, 1, B->st);
 }
 
+static void batch_level_op(Batch* B, int l, bool correct) {
+    for (const bool split : {true, false}) {
+        const LaunchList& L = split ? B->lsp[l] : B->lnd[l];
+        if (L.n) launch_batch_level_op32(args_of<BatchLevelOp>(L), L.act, L.n, split, correct, B->st);
+    }
+}
+
 static void batch_product(Batch* B, int mode, const LaunchList& L) {
     launch_batch_matvec32(B->variant, mode, args_of<BatchMatvec>(L), L.act, L.n, B->kh, B->mv_grid, B->err, B->st);
 }
@@ -408,17 +420,16 @@ static void batch_vcycle(Batch* B) {
         return;
     }
     for (int l = 0; l + 1 < B->maxL; ++l) {
-        const LaunchList& op = B->lop[l];
-        if (l == 0) batch_product(B, 1, B->mv1);                                                     // t = r - K x
-        else if (op.n) launch_batch_level_op32(args_of<BatchLevelOp>(op), op.act, op.n, false, B->st);
+        if (l == 0) batch_product(B, 1, B->mv1);                       // t = r - K x
+        else batch_level_op(B, l, false);
         batch_restrict(B, l);                                          // r' = P^T t, x' = w r' / D'
     }
     launch_batch_coarse32(args_of<BatchCoarse>(B->co), B->co.act, B->co.n, B->coarse_max, B->st);
     for (int l = B->maxL - 2; l >= 1; --l) {
-        const LaunchList &pa = B->pa[l], &op = B->lop[l];
+        const LaunchList& pa = B->pa[l];
         if (!pa.n) continue;
         launch_batch_prolong_add32(args_of<BatchProlongAdd>(pa), pa.act, pa.n, B->st);        // x += P x'
-        launch_batch_level_op32(args_of<BatchLevelOp>(op), op.act, op.n, true, B->st);        // t = x + w (r - K x) / D
+        batch_level_op(B, l, true);                                                           // t = x + w (r - K x) / D
     }
     launch_batch_prolong_add32(args_of<BatchProlongAdd>(B->pa[0]), B->pa[0].act, B->pa[0].n, B->st);   // T = z + P x'
     batch_product(B, 2, B->mv2);                                      // z = T + w (r - K T) / D, with r.z

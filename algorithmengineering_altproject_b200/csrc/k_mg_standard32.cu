@@ -302,6 +302,20 @@ __global__ void __launch_bounds__(LS_THREADS, 1) k_level_split32(MgLevel32 L, co
     level_split32<OP>(vb_real(), L, Kel, x, r, y, w, S, sp, sums);
 }
 template <LevelOp OP>
+__device__ __forceinline__ void level_nodes32(VB vb, const MgLevel32& L, const float* __restrict__ Kel,
+                                              const float* __restrict__ x, const float* __restrict__ r,
+                                              float* __restrict__ y, float w, const PcgScalars* S,
+                                              const SymPositions& sp) {
+    if (S->done) return;
+    const int ne = L.nx * L.ny * L.nz;
+    const int64_t n = (int64_t)vb.b * LN_NODES + threadIdx.x;
+    if (n >= L.nn) return;
+    float kx[3];
+    level_nodes<3, float>(L, L.cs, (int)n, 0, Kel, x, [&](int i, auto&& take) { sp.row(i, ne, take); }, kx);
+#pragma unroll
+    for (int row = 0; row < 3; ++row) level_store32<OP>(L, (int)n, row, kx[row], x, r, y, w);
+}
+template <LevelOp OP>
 __global__ void __launch_bounds__(LN_NODES, 3) k_level_nodes32(MgLevel32 L, const float* __restrict__ Kel,
                                                                  const float* __restrict__ x,
                                                                  const float* __restrict__ r, float* __restrict__ y,
@@ -309,13 +323,7 @@ __global__ void __launch_bounds__(LN_NODES, 3) k_level_nodes32(MgLevel32 L, cons
     __shared__ SymPositions sp;
     if (S->done) return;
     sp.fill();
-    const int ne = L.nx * L.ny * L.nz;
-    const int64_t n = (int64_t)blockIdx.x * LN_NODES + threadIdx.x;
-    if (n >= L.nn) return;
-    float kx[3];
-    level_nodes<3, float>(L, L.cs, (int)n, 0, Kel, x, [&](int i, auto&& take) { sp.row(i, ne, take); }, kx);
-#pragma unroll
-    for (int row = 0; row < 3; ++row) level_store32<OP>(L, (int)n, row, kx[row], x, r, y, w);
+    level_nodes32<OP>(vb_real(), L, Kel, x, r, y, w, S, sp);
 }
 // nodes up to which the split form is used: four waves of its blocks (one per SM).  Measured at 9,537 nodes in FP32:
 // a V-cycle at 256x512x256 2.45 ms split, 2.48 not; at 30,625: 35 us split, 22 not (FP64: 0.764 against 0.731 ms a cycle).
@@ -380,8 +388,8 @@ __global__ void __launch_bounds__(256) k_batch_prolong_add32(const BatchProlongA
     });
 }
 template <LevelOp OP>
-__global__ void __launch_bounds__(LS_THREADS, 1) k_batch_level_op32(const BatchLevelOp* __restrict__ a,
-                                                                    const int* __restrict__ act, int N) {
+__global__ void __launch_bounds__(LS_THREADS, 1) k_batch_level_split32(const BatchLevelOp* __restrict__ a,
+                                                                       const int* __restrict__ act, int N) {
     __shared__ SymPositions sp;
     __shared__ float sums[3 * LS_NODES];
     sp.fill();
@@ -390,18 +398,38 @@ __global__ void __launch_bounds__(LS_THREADS, 1) k_batch_level_op32(const BatchL
         level_split32<OP>(vb, L, A.Kel, A.x, A.r, A.y, A.w, A.S, sp, sums);
     });
 }
-constexpr int BATCH_GRID256 = 8 * 148, BATCH_GRID_LS = 148;
+template <LevelOp OP>
+__global__ void __launch_bounds__(LN_NODES, 3) k_batch_level_nodes32(const BatchLevelOp* __restrict__ a,
+                                                                     const int* __restrict__ act, int N) {
+    __shared__ SymPositions sp;
+    sp.fill();
+    batch_walk(a, act, N, [&](const BatchLevelOp& A, VB vb) {
+        const MgLevel32 L = A.L;
+        level_nodes32<OP>(vb, L, A.Kel, A.x, A.r, A.y, A.w, A.S, sp);
+    });
+}
+constexpr int BATCH_GRID256 = 8 * 148, BATCH_GRID_LS = 148, BATCH_GRID_LN = 3 * 148;
 
 }  // namespace
 
 int batch_blocks_prolong_add(const BatchProlongAdd& a) { return (int)blocks_of(a.Lf.nn, 256); }
-int batch_blocks_level_op(const BatchLevelOp& a) { return (int)blocks_of(a.L.nn, LS_NODES); }
+// Each member's level takes the form of its solo launch, for the same reason.  All levels split against this rule, ms an
+// iteration: two members of 96x192x96 0.85, 0.77; one of 192x384x192 2.05, 1.70 (alone 1.61).
+bool batch_level_split(const BatchLevelOp& a) { return a.L.nn <= LEVEL_SPLIT_MAX32; }
+int batch_blocks_level_op(const BatchLevelOp& a) {
+    return (int)blocks_of(a.L.nn, batch_level_split(a) ? LS_NODES : LN_NODES);
+}
 void launch_batch_prolong_add32(const BatchProlongAdd* a, const int* act, int N, cudaStream_t s) {
     k_batch_prolong_add32<<<BATCH_GRID256, 256, 0, s>>>(a, act, N);
 }
-void launch_batch_level_op32(const BatchLevelOp* a, const int* act, int N, bool correct, cudaStream_t s) {
-    if (correct) k_batch_level_op32<LevelOp::Correct><<<BATCH_GRID_LS, LS_THREADS, 0, s>>>(a, act, N);
-    else k_batch_level_op32<LevelOp::Residual><<<BATCH_GRID_LS, LS_THREADS, 0, s>>>(a, act, N);
+void launch_batch_level_op32(const BatchLevelOp* a, const int* act, int N, bool split, bool correct, cudaStream_t s) {
+    if (split) {
+        if (correct) k_batch_level_split32<LevelOp::Correct><<<BATCH_GRID_LS, LS_THREADS, 0, s>>>(a, act, N);
+        else k_batch_level_split32<LevelOp::Residual><<<BATCH_GRID_LS, LS_THREADS, 0, s>>>(a, act, N);
+        return;
+    }
+    if (correct) k_batch_level_nodes32<LevelOp::Correct><<<BATCH_GRID_LN, LN_NODES, 0, s>>>(a, act, N);
+    else k_batch_level_nodes32<LevelOp::Residual><<<BATCH_GRID_LN, LN_NODES, 0, s>>>(a, act, N);
 }
 
 void launch_jacobi_init32(const MgLevel32& L, const float* r, float* x, float w, const PcgScalars* S, cudaStream_t s) {

@@ -405,9 +405,10 @@ struct BatchLevelOp {     // y = r - K_l x, or y = x + w (r - K_l x) / D, from t
     PcgScalars* S;
 };
 int batch_blocks_prolong_add(const BatchProlongAdd& a);
+bool batch_level_split(const BatchLevelOp& a);   // the form its level takes (a launch holds members of one form)
 int batch_blocks_level_op(const BatchLevelOp& a);
 void launch_batch_prolong_add32(const BatchProlongAdd* a, const int* act, int N, cudaStream_t s);
-void launch_batch_level_op32(const BatchLevelOp* a, const int* act, int N, bool correct, cudaStream_t s);
+void launch_batch_level_op32(const BatchLevelOp* a, const int* act, int N, bool split, bool correct, cudaStream_t s);
 
 struct BatchCompact {     // one launch list's compaction: act from the done flags of its N instances
     PcgScalars* const* S;   // per position
