@@ -86,12 +86,14 @@ constexpr int KE_MAX_DISTINCT = 32;   // room for the distinct-magnitude list of
 // distinct magnitudes (the streaming kernel's register-operand form)
 bool ke_pattern_magnitudes(const double* Ke, double* D);
 int stream64_tiling(const Grid& g, int dev, Stream64Tiling* t);
+// the residual and correction kernels' part of it: shared-memory attribute set, resident CTAs per SM (at least)
+int stream64_occupancy_residual(int* per_sm);
+int stream64_occupancy_correct(int* per_sm);
 // Kd: device copy of the magnitudes when Ke has the built-in pattern, else nullptr; then Ke_host (the
 // context's host copy of Ke) is copied into the launch (and into a graph that captures it)
 void launch_matvec64_stream(const Grid& g, const Stream64Tiling& t, const double* Ke_host, const double* Kd,
                             const double* E, const uint8_t* mask, const double* u, double* y, const PcgScalars* S,
                             cudaStream_t s);
-// S->denom = p.Ap (3 components) in the canonical reduction order, unless S->done
 // the same with the Standard V-cycle's step: y = r - K u, and y = u + w (r - K u) / D (y other than u)
 void launch_residual64_stream(const Grid& g, const Stream64Tiling& t, const double* Ke_host, const double* Kd,
                               const double* E, const uint8_t* mask, const double* u, const double* r, double* y,
@@ -99,6 +101,7 @@ void launch_residual64_stream(const Grid& g, const Stream64Tiling& t, const doub
 void launch_correct64_stream(const Grid& g, const Stream64Tiling& t, const double* Ke_host, const double* Kd,
                              const double* E, const uint8_t* mask, const double* u, const double* r, const double* diag,
                              double w, double* y, const PcgScalars* S, cudaStream_t s);
+// S->denom = p.Ap (3 components) in the canonical reduction order, unless S->done
 void launch_dot_pcg(const Grid& g, const double* p, const double* Ap, RedSlot red, PcgScalars* S, cudaStream_t s);
 void launch_compliance64(const Grid& g, const double* Ke, const double* E, const double* u, double* ce,
                          RedSlot red, double* C, cudaStream_t s);
