@@ -142,6 +142,7 @@ static int build_levels(Context* c) {
     for (int l = 0; l + 1 < c->nlev; ++l) {
         const MgLevel &Lf = c->lv[l], &Lc = c->lv[l + 1];
         CHECK(c->alloc(&c->ra1[l], (size_t)3 * (Lf.nz + 1) * (Lf.ny + 1) * (Lc.nx + 1)));
+        if (restrict_by_axes(Lc)) CHECK(c->alloc(&c->ra2, (size_t)3 * (Lf.nz + 1) * (Lc.ny + 1) * (Lc.nx + 1)));
     }
     T3D_CUDA_OK(mg_kernel_attributes());
     CHECK(c->alloc(&c->chol_status, 1));
@@ -693,7 +694,7 @@ static void vcycle_standard(Context* c, const double* r, double* z, PcgScalars* 
     for (int l = 0; l + 1 < L; ++l) {
         const MgLevel &Lf = c->lv[l], &Lc = c->lv[l + 1];
         if (l > 0) launch_level_op(Lf, c->KelT[l], Lf.x, Lf.r, c->vtmp[l], false, w, S, c->st);
-        launch_restrict(Lc, Lf, l == 0 ? c->Ap : c->vtmp[l], Lc.r, c->ra1[l], S, c->st, false,
+        launch_restrict(Lc, Lf, l == 0 ? c->Ap : c->vtmp[l], Lc.r, c->ra1[l], c->ra2, S, c->st, false,
                         l + 2 < L ? Lc.x : nullptr, w);
     }
     launch_coarse_solve(c->lv[L - 1], c->Xc, c->Nc, c->chol_status, S, c->st);
@@ -718,7 +719,7 @@ static void vcycle(Context* c, const double* r, double* z, PcgScalars* S, RedSlo
     const int L = c->nlev, tail = adapted_tail_first(c->lv, L, c->Nc), down = std::min(tail, L - 1);
     c->launches += vcycle_launches(c);
     for (int l = 0; l < down; ++l)
-        launch_restrict(c->lv[l + 1], c->lv[l], l == 0 ? r : c->lv[l].r, c->lv[l + 1].r, c->ra1[l], S, c->st);
+        launch_restrict(c->lv[l + 1], c->lv[l], l == 0 ? r : c->lv[l].r, c->lv[l + 1].r, c->ra1[l], c->ra2, S, c->st);
     if (tail < L)
         launch_adapted_tail(c->lv, L, tail, c->Xc, c->Nc, c->chol_status, (double)c->prm.mg_weight, S, c->st);
     else

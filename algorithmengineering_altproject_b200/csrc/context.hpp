@@ -72,6 +72,7 @@ struct Context {
     RedSlot slot[4]{};
     double *Kce = nullptr, *Kc = nullptr, *LT = nullptr, *Lrow = nullptr, *Xc = nullptr;
     double* ra1[8]{};           // x-pass buffer of the separable restriction per level transition
+    double* ra2 = nullptr;      // y-pass buffer of a large first transition (restrict_by_axes)
     int* chol_status = nullptr;
     double *frhs = nullptr, *fx = nullptr, *fr = nullptr, *fz = nullptr, *fp = nullptr, *fAp = nullptr,
            *flastx = nullptr, *flastrhs = nullptr, *fdiag = nullptr;

@@ -210,6 +210,54 @@ __global__ void __launch_bounds__(128) k_restrict_yz(MgLevel Lc, MgLevel Lf, con
     restrict_store(Lc, n, c, restrict_scale(Lc, Lf, n, cx, cy, cz, c, v, normalize), rc, x0, w0);
 }
 
+// The same two sums as separate passes, for large coarse grids: the y sum of every fine z once (a2: fine z x coarse y x
+// coarse x), instead of once for each of the two coarse z whose windows hold it.  a, a2: one component (blockIdx.y).
+template <int SP>
+__global__ void __launch_bounds__(256) k_restrict_y(MgLevel Lc, MgLevel Lf, const double* __restrict__ a1,
+                                                    double* __restrict__ a2, const PcgScalars* S) {
+    if (S != nullptr && S->done) return;
+    constexpr int WS = 2 * SP - 1;
+    const int cnx = Lc.nx + 1, cny = Lc.ny + 1, fny = Lf.ny + 1, fnz = Lf.nz + 1, n2 = fnz * cny * cnx;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
+    if (i >= n2) return;
+    const int cx = i % cnx, cy = (i / cnx) % cny, fz = i / (cnx * cny);
+    const double* __restrict__ a = a1 + c * ((int64_t)fnz * fny * cnx) + cx;
+    double q[WS];
+#pragma unroll
+    for (int iy = 0; iy < WS; ++iy) {
+        const int fy = cy * SP + iy - (SP - 1);
+        q[iy] = fy >= 0 && fy < fny ? a[(fz * fny + fy) * cnx] : 0.0;
+    }
+    double t = 0.0;
+#pragma unroll
+    for (int iy = 0; iy < WS; ++iy) t = t + hat(iy, SP) * q[iy];
+    a2[(int64_t)c * n2 + i] = t;
+}
+template <int SP>
+__global__ void __launch_bounds__(128) k_restrict_z(MgLevel Lc, MgLevel Lf, const double* __restrict__ a2,
+                                                    double* __restrict__ rc, const PcgScalars* S, int normalize,
+                                                    double* __restrict__ x0, double w0) {
+    if (S != nullptr && S->done) return;
+    constexpr int WS = 2 * SP - 1;
+    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= Lc.nn) return;
+    const int cnx = Lc.nx + 1, cny = Lc.ny + 1, fnz = Lf.nz + 1;
+    const int cx = n % cnx, cy = (n / cnx) % cny, cz = n / (cnx * cny);
+    const int64_t n2 = (int64_t)fnz * cny * cnx;
+    const double* __restrict__ a = a2 + cy * cnx + cx;
+    double v[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int iz = 0; iz < WS; ++iz) {
+        const int fz = cz * SP + iz - (SP - 1);
+        const bool in = fz >= 0 && fz < fnz;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) v[c] = v[c] + hat(iz, SP) * (in ? a[c * n2 + fz * cny * cnx] : 0.0);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+        restrict_store(Lc, n, c, restrict_scale(Lc, Lf, n, cx, cy, cz, c, v[c], normalize), rc, x0, w0);
+}
+
 // The 27-point window of a span-2 transition in the same nested order, from one component's residual
 __device__ __forceinline__ double window2(const MgLevel& Lc, const MgLevel& Lf, int cx, int cy, int cz,
                                           const double* rf) {
@@ -282,17 +330,24 @@ __device__ __forceinline__ double smooth(double w, double r, double d, double P,
     return fixed ? 0.0 : (t + P) + t;
 }
 
-// one thread per node and component (blockIdx.y)
-__global__ void __launch_bounds__(128) k_prolong_smooth(MgLevel Lc, MgLevel Lf, const double* __restrict__ xc,
-                                                        const double* __restrict__ rf, double* __restrict__ xf,
-                                                        double w, const PcgScalars* S) {
+// COMPS components of a node per thread (3 / COMPS blocks in y)
+template <int COMPS>
+__global__ void __launch_bounds__(COMPS == 1 ? 128 : 256) k_prolong_smooth(MgLevel Lc, MgLevel Lf,
+                                                                           const double* __restrict__ xc,
+                                                                           const double* __restrict__ rf,
+                                                                           double* __restrict__ xf, double w,
+                                                                           const PcgScalars* S) {
     if (S != nullptr && S->done) return;
-    const int n = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
+    const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= Lf.nn) return;
     const int fnx = Lf.nx + 1, fny = Lf.ny + 1;
     const ProlongAt P(Lc, Lc.span, n % fnx, (n / fnx) % fny, n / (fnx * fny));
-    const int64_t i = c * Lf.nn + n;
-    xf[i] = smooth(w, rf[i], Lf.diag[i], P(xc + c * Lc.nn), (Lf.mask[n] >> c) & 1);
+#pragma unroll
+    for (int k = 0; k < COMPS; ++k) {
+        const int c = COMPS * blockIdx.y + k;
+        const int64_t i = c * Lf.nn + n;
+        xf[i] = smooth(w, rf[i], Lf.diag[i], P(xc + c * Lc.nn), (Lf.mask[n] >> c) & 1);
+    }
 }
 
 // level 0: writes z and forms r.z in the canonical order; the last block sets rz (first use) or
@@ -306,11 +361,13 @@ __global__ void __launch_bounds__(RED_THREADS) k_prolong_smooth0(MgLevel Lc, MgL
     const int fnx = Lf.nx + 1, fny = Lf.ny + 1;
     double part = 0.0;
     for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < NN; n += gridDim.x * blockDim.x) {
-        const ProlongAt P(Lc, Lc.span, n % fnx, (n / fnx) % fny, n / (fnx * fny));
+        const ProlongAt at(Lc, Lc.span, n % fnx, (n / fnx) % fny, n / (fnx * fny));
+        double P[3];   // the coarse corners first: their loads together, ahead of the fine node's
+        for (int c = 0; c < 3; ++c) P[c] = at(xc + c * Lc.nn);
         const int m = Lf.mask[n];
         for (int c = 0; c < 3; ++c) {
             const double rv = r[c * (int64_t)NN + n];
-            const double zv = smooth(w, rv, Lf.diag[c * (int64_t)NN + n], P(xc + c * Lc.nn), (m >> c) & 1);
+            const double zv = smooth(w, rv, Lf.diag[c * (int64_t)NN + n], P[c], (m >> c) & 1);
             z[c * (int64_t)NN + n] = zv;
             part = part + rv * zv;
         }
@@ -729,9 +786,14 @@ void launch_mask_restrict(const MgLevel& Lc, const MgLevel& Lf, cudaStream_t s) 
 void launch_diag_coarsen(const MgLevel& Lc, const MgLevel& Lf, cudaStream_t s) {
     k_diag_coarsen<<<dim3(blocks_for(Lc.nn, 64), 3), 64, 0, s>>>(Lc, Lf);
 }
-// span 4 (the first transition): x pass, then the y-z pass; span 2: the whole window.  A separate y pass reads
-// less, and its two launches cost more up to about 10^5 coarse nodes.
-void launch_restrict(const MgLevel& Lc, const MgLevel& Lf, const double* rf, double* rc, double* a1,
+// Levels of more nodes take fewer operations a node: separate y and z passes, and one thread for a node's three
+// components.  Below, more threads with less work each finish sooner.  An Adapted V-cycle with all levels in the first
+// and in the second form, ms: 0.264 and 0.261 at 70,785 level-1 nodes, 0.419 and 0.428 at 136,161, 0.662 and 0.682 at
+// 232,897, 1.467 and 1.525 at 545,025.
+constexpr int64_t LARGE_LEVEL = 100000;
+
+// span 4 (the first transition): x pass, then the y-z pass or separate y and z passes; span 2: the whole window.
+void launch_restrict(const MgLevel& Lc, const MgLevel& Lf, const double* rf, double* rc, double* a1, double* a2,
                      const PcgScalars* S, cudaStream_t s, bool normalize, double* x0, double w) {
     const dim3 b(blocks_for(Lc.nn, 128), 3);
     if (Lc.span == 2) {
@@ -740,12 +802,22 @@ void launch_restrict(const MgLevel& Lc, const MgLevel& Lf, const double* rf, dou
     }
     const int64_t n1 = (int64_t)(Lf.nz + 1) * (Lf.ny + 1) * (Lc.nx + 1);
     k_restrict_x<<<blocks_for(n1, 256), 256, 0, s>>>(Lc, Lf, rf, a1, S);
-    k_restrict_yz<4><<<b, 128, 0, s>>>(Lc, Lf, a1, rc, S, normalize ? 1 : 0, x0, w);
+    if (!restrict_by_axes(Lc)) {
+        k_restrict_yz<4><<<b, 128, 0, s>>>(Lc, Lf, a1, rc, S, normalize ? 1 : 0, x0, w);
+        return;
+    }
+    const int64_t n2 = (int64_t)(Lf.nz + 1) * (Lc.ny + 1) * (Lc.nx + 1);
+    k_restrict_y<4><<<dim3(blocks_for(n2, 256), 3), 256, 0, s>>>(Lc, Lf, a1, a2, S);
+    k_restrict_z<4><<<b.x, 128, 0, s>>>(Lc, Lf, a2, rc, S, normalize ? 1 : 0, x0, w);
 }
-int restrict_launches(const MgLevel& Lc) { return Lc.span == 2 ? 1 : 2; }
+bool restrict_by_axes(const MgLevel& Lc) { return Lc.span == 4 && Lc.nn > LARGE_LEVEL; }
+int restrict_launches(const MgLevel& Lc) { return Lc.span == 2 ? 1 : restrict_by_axes(Lc) ? 3 : 2; }
 void launch_prolong_smooth(const MgLevel& Lc, const MgLevel& Lf, const double* xc, const double* rf, double* xf,
                            double weight, const PcgScalars* S, cudaStream_t s) {
-    k_prolong_smooth<<<dim3(blocks_for(Lf.nn, 128), 3), 128, 0, s>>>(Lc, Lf, xc, rf, xf, weight, S);
+    if (Lf.nn <= LARGE_LEVEL)
+        k_prolong_smooth<1><<<dim3(blocks_for(Lf.nn, 128), 3), 128, 0, s>>>(Lc, Lf, xc, rf, xf, weight, S);
+    else
+        k_prolong_smooth<3><<<blocks_for(Lf.nn, 256), 256, 0, s>>>(Lc, Lf, xc, rf, xf, weight, S);
 }
 void launch_prolong_smooth0(const MgLevel& Lc, const MgLevel& Lf, const double* xc, const double* r, double* z,
                             double weight, RedSlot dot, PcgScalars* S, cudaStream_t s) {

@@ -119,9 +119,12 @@ void launch_diag0(const Grid& g, const double* Ke, const double* E, const uint8_
                   cudaStream_t s);
 void launch_mask_restrict(const MgLevel& Lc, const MgLevel& Lf, cudaStream_t s);
 void launch_diag_coarsen(const MgLevel& Lc, const MgLevel& Lf, cudaStream_t s);
-// separable restriction; a1, a2: pass buffers of 3*(fnz*fny*cnx) and 3*(fnz*cny*cnx) doubles
-// normalize = false: the transpose of the trilinear prolongation (no division by the weight sum)
-void launch_restrict(const MgLevel& Lc, const MgLevel& Lf, const double* rf, double* rc, double* a1,
+// separable restriction; a1: the x pass's 3*(fnz*fny*cnx) doubles on a span-4 transition (else unused), a2: the y
+// pass's 3*(fnz*cny*cnx) where restrict_by_axes says that there is one
+// normalize = false: the transpose of the trilinear prolongation (no division by the weight sum); with x0, the
+// coarse level's Jacobi start x0 = w rc / D is written too
+bool restrict_by_axes(const MgLevel& Lc);
+void launch_restrict(const MgLevel& Lc, const MgLevel& Lf, const double* rf, double* rc, double* a1, double* a2,
                      const PcgScalars* S, cudaStream_t s, bool normalize = true,
                      double* x0 = nullptr, double w = 0.0);
 void launch_prolong_smooth(const MgLevel& Lc, const MgLevel& Lf, const double* xc, const double* rf, double* xf,
