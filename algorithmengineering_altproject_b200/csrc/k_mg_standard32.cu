@@ -325,10 +325,46 @@ __global__ void __launch_bounds__(LN_NODES, 3) k_level_nodes32(MgLevel32 L, cons
     sp.fill();
     level_nodes32<OP>(vb_real(), L, Kel, x, r, y, w, S, sp);
 }
-// nodes up to which the split form is used: four waves of its blocks (one per SM).  Measured at 9,537 nodes in FP32:
-// a V-cycle at 256x512x256 2.45 ms split, 2.48 not; at 30,625: 35 us split, 22 not (FP64: 0.764 against 0.731 ms a cycle).
-constexpr int64_t LEVEL_SPLIT_MAX32 = 4 * 148 * LS_NODES;
-
+// The third form, for the largest levels: a thread per node, the loops unrolled over all elements and columns, so that
+// the packed positions are constants and a load is an address away from the last one.
+template <LevelOp OP>
+__device__ __forceinline__ void level_unrolled32(VB vb, const MgLevel32& L, const float* __restrict__ Kel,
+                                                 const float* __restrict__ x, const float* __restrict__ r,
+                                                 float* __restrict__ y, float w, const PcgScalars* S) {
+    if (S->done) return;
+    const int64_t n = (int64_t)vb.b * LN_NODES + threadIdx.x;
+    if (n >= L.nn) return;
+    const int nnx = L.nx + 1, nny = L.ny + 1;
+    const int64_t ne = (int64_t)L.nx * L.ny * L.nz;
+    const int X = (int)n % nnx, Y = ((int)n / nnx) % nny, Z = (int)n / (nnx * nny);
+    float kx[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const LpElement el(L.nx, L.ny, L.nz, X, Y, Z, q);
+        if (!el.in) continue;
+        const float* __restrict__ K = Kel + el.e;
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+            const float* __restrict__ p = x + el.m + (corner_dz(b) * nny + corner_dy(b)) * nnx + corner_dx(b);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const float xv = p[c * L.cs];
+#pragma unroll
+                for (int row = 0; row < 3; ++row)
+                    kx[row] = lp_add(kx[row], K[sym_pack(3 * corner_of(q & 1, (q >> 1) & 1, q >> 2) + row, 3 * b + c) * ne], xv);
+            }
+        }
+    }
+#pragma unroll
+    for (int row = 0; row < 3; ++row) level_store32<OP>(L, (int)n, row, kx[row], x, r, y, w);
+}
+template <LevelOp OP>
+__global__ void __launch_bounds__(LN_NODES) k_level_unrolled32(MgLevel32 L, const float* __restrict__ Kel,
+                                                               const float* __restrict__ x,
+                                                               const float* __restrict__ r, float* __restrict__ y,
+                                                               float w, const PcgScalars* S) {
+    level_unrolled32<OP>(vb_real(), L, Kel, x, r, y, w, S);
+}
 // FP32 symmetric-packed, entry-major image of element-major FP64 element matrices (the upper triangle):
 // dst[p * ne + e] = src[e * 576 + 24 i + j], (i, j) the p-th upper-triangle entry
 __global__ void k_kel_pack32(int64_t ne, const double* __restrict__ src, float* __restrict__ dst) {
@@ -412,24 +448,34 @@ constexpr int BATCH_GRID256 = 8 * 148, BATCH_GRID_LS = 148, BATCH_GRID_LN = 3 * 
 
 }  // namespace
 
+// The form by the level's nodes.  Split up to four waves of its blocks (one per SM): 2.45 against 2.48 ms for a V-cycle at
+// 256x512x256 with its 9,537-node level in the other form; at 30,625 nodes the product takes 35 us split, 22 by nodes.
+// Unrolled above 50,000: a V-cycle takes 0.245 ms with 30,625 nodes unrolled and 0.235 not, with 70,785 0.431 and 0.445,
+// with 545,025 2.10 and 2.17.
+enum class LevelForm32 { Split, Nodes, Unrolled };
+static LevelForm32 level_form32(int64_t nn) {
+    return nn <= 4 * 148 * LS_NODES ? LevelForm32::Split : nn <= 50000 ? LevelForm32::Nodes : LevelForm32::Unrolled;
+}
+
 int batch_blocks_prolong_add(const BatchProlongAdd& a) { return (int)blocks_of(a.Lf.nn, 256); }
-// Each member's level takes the form of its solo launch, for the same reason.  All levels split against this rule, ms an
-// iteration: two members of 96x192x96 0.85, 0.77; one of 192x384x192 2.05, 1.70 (alone 1.61).
-bool batch_level_split(const BatchLevelOp& a) { return a.L.nn <= LEVEL_SPLIT_MAX32; }
+// A member's level is split up to the same size as alone.  All levels split, and by this rule, ms an iteration: two members
+// of 96x192x96 0.85, 0.77; one of 192x384x192 2.05, 1.70.  Above it the rolled form: unrolled it is no faster here (two of
+// 160x320x160 2.19 against 2.18).
+bool batch_level_split(const BatchLevelOp& a) { return level_form32(a.L.nn) == LevelForm32::Split; }
 int batch_blocks_level_op(const BatchLevelOp& a) {
     return (int)blocks_of(a.L.nn, batch_level_split(a) ? LS_NODES : LN_NODES);
 }
 void launch_batch_prolong_add32(const BatchProlongAdd* a, const int* act, int N, cudaStream_t s) {
     k_batch_prolong_add32<<<BATCH_GRID256, 256, 0, s>>>(a, act, N);
 }
+template <LevelOp OP>
+static void batch_level_op(const BatchLevelOp* a, const int* act, int N, bool split, cudaStream_t s) {
+    if (split) k_batch_level_split32<OP><<<BATCH_GRID_LS, LS_THREADS, 0, s>>>(a, act, N);
+    else k_batch_level_nodes32<OP><<<BATCH_GRID_LN, LN_NODES, 0, s>>>(a, act, N);
+}
 void launch_batch_level_op32(const BatchLevelOp* a, const int* act, int N, bool split, bool correct, cudaStream_t s) {
-    if (split) {
-        if (correct) k_batch_level_split32<LevelOp::Correct><<<BATCH_GRID_LS, LS_THREADS, 0, s>>>(a, act, N);
-        else k_batch_level_split32<LevelOp::Residual><<<BATCH_GRID_LS, LS_THREADS, 0, s>>>(a, act, N);
-        return;
-    }
-    if (correct) k_batch_level_nodes32<LevelOp::Correct><<<BATCH_GRID_LN, LN_NODES, 0, s>>>(a, act, N);
-    else k_batch_level_nodes32<LevelOp::Residual><<<BATCH_GRID_LN, LN_NODES, 0, s>>>(a, act, N);
+    if (correct) batch_level_op<LevelOp::Correct>(a, act, N, split, s);
+    else batch_level_op<LevelOp::Residual>(a, act, N, split, s);
 }
 
 void launch_jacobi_init32(const MgLevel32& L, const float* r, float* x, float w, const PcgScalars* S, cudaStream_t s) {
@@ -446,17 +492,19 @@ void launch_prolong_add32(const MgLevel32& Lc, const MgLevel32& Lf, const float*
                           const PcgScalars* S, cudaStream_t s) {
     k_prolong_add32<<<blocks_of(Lf.nn, 256), 256, 0, s>>>(Lc, Lf, xc, xi, xo, S);
 }
+template <LevelOp OP>
+static void level_op(const MgLevel32& L, const float* Kel, const float* x, const float* r, float* y, float w,
+                     const PcgScalars* S, cudaStream_t s) {
+    const LevelForm32 form = level_form32(L.nn);
+    const unsigned b = blocks_of(L.nn, form == LevelForm32::Split ? LS_NODES : LN_NODES);
+    if (form == LevelForm32::Split) k_level_split32<OP><<<b, LS_THREADS, 0, s>>>(L, Kel, x, r, y, w, S);
+    else if (form == LevelForm32::Nodes) k_level_nodes32<OP><<<b, LN_NODES, 0, s>>>(L, Kel, x, r, y, w, S);
+    else k_level_unrolled32<OP><<<b, LN_NODES, 0, s>>>(L, Kel, x, r, y, w, S);
+}
 void launch_level_op32(const MgLevel32& L, const float* Kel, const float* x, const float* r, float* y, bool correct,
                        float w, const PcgScalars* S, cudaStream_t s) {
-    if (L.nn <= LEVEL_SPLIT_MAX32) {
-        const unsigned b = blocks_of(L.nn, LS_NODES);
-        if (correct) k_level_split32<LevelOp::Correct><<<b, LS_THREADS, 0, s>>>(L, Kel, x, r, y, w, S);
-        else k_level_split32<LevelOp::Residual><<<b, LS_THREADS, 0, s>>>(L, Kel, x, r, y, w, S);
-        return;
-    }
-    const unsigned b = (unsigned)((L.nn + LN_NODES - 1) / LN_NODES);
-    if (correct) k_level_nodes32<LevelOp::Correct><<<b, LN_NODES, 0, s>>>(L, Kel, x, r, y, w, S);
-    else k_level_nodes32<LevelOp::Residual><<<b, LN_NODES, 0, s>>>(L, Kel, x, r, y, w, S);
+    if (correct) level_op<LevelOp::Correct>(L, Kel, x, r, y, w, S, s);
+    else level_op<LevelOp::Residual>(L, Kel, x, r, y, w, S, s);
 }
 void launch_kel_pack32(int64_t ne, const double* Kel, float* KelP32, cudaStream_t s) {
     k_kel_pack32<<<(unsigned)((ne + 31) / 32), dim3(32, 8), 0, s>>>(ne, Kel, KelP32);

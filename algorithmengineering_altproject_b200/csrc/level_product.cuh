@@ -8,12 +8,15 @@
 //   level_split  small levels, latency-bound: a block is 32 nodes x 3 rows x 8 elements (a warp per row and
 //                element), so all 192 loads of a row are in flight at once; the eight warps of a row then add
 //                their 24 columns one after the other, handing the running sum on through shared memory.
-//   level_nodes  large levels, bound by the matrices' L2 and DRAM traffic: a thread per node with ROWS of its rows
-//                (3 in FP32; 1 in FP64, the other rows in the block's other warps), a rolled loop over the elements.  (Unrolled over all elements the code, 50 KB, ran at the rate
-//                of instruction-cache misses: 6 of 8 stall cycles per instruction.)
-// Both add in the same order: identical bits.  Against a thread per node, fully unrolled, and separate residual and
+//   level_nodes  larger levels, bound by the matrices' L2 and DRAM traffic: a thread per node with ROWS of its rows
+//                (3 in FP32; 1 in FP64, the other rows in the block's other warps), a rolled loop over the elements.
+//                (Unrolled over all elements the code, 50 KB, runs at the rate of instruction-cache misses at 30,625
+//                nodes: 6 of 8 stall cycles per instruction.  The FP32 product is unrolled all the same on the largest
+//                levels, k_mg_standard32.cu.)
+// All add in the same order: identical bits.  Against a thread per node, fully unrolled, and separate residual and
 // correction passes (ncu, cold caches): FP32 25 + 4 -> 7 us at 4,225 nodes, 31 + 6 -> 22 us at 30,625; FP64 57 + 6
-// -> 9 us at 4,225.  A V-cycle: FP32 0.386 -> 0.277 ms at 96x192x96, FP64 0.338 -> 0.251 ms at 48x96x48.
+// -> 9 us at 4,225, 433 + 9 -> 409 us at 545,025.  A V-cycle: FP32 0.386 -> 0.277 ms at 96x192x96, FP64 0.338 -> 0.251
+// ms at 48x96x48.
 #pragma once
 #include "t3d_common.cuh"
 
