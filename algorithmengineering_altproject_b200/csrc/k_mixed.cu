@@ -219,45 +219,59 @@ __device__ __forceinline__ void restrict_store32(const MgLevel32& Lc, const MgLe
     if (x0) x0[i] = fixed ? 0.0f : (w0 * o) * Lc.diag[i];
 }
 
+// A V-cycle with the y-z pass's three components in three threads and in one, ms: 0.1455 and 0.1475 with 9,537 coarse
+// nodes, equal at 70,785, 1.011 and 1.007 at 232,897, 2.098 and 2.090 at 545,025 (the pass 48 and 36 us).
+constexpr int64_t RESTRICT32_LARGE = 100000;
+
 // The transfers below take one thread per coarse node and component (component-major); points outside the grid load
 // nothing and add +0, which changes no sum, so that all loads of a window row are in flight together.
-// y and z window sums of the x-pass result a1[fz][fy][cx] in one pass.
-template <int SP>
+// y and z window sums of the x-pass result a1[fz][fy][cx] in one pass; COMPS components of a node per thread.
+template <int SP, int COMPS>
 __device__ __forceinline__ void restrict_yz32(VB vb, const MgLevel32& Lc, const MgLevel32& Lf,
                                               const float* __restrict__ a1, float* __restrict__ rc,
                                               const PcgScalars* S, int normalize, float* __restrict__ x0, float w0) {
     if (S->done) return;
     constexpr int WS = 2 * SP - 1;
     const int i = vb.b * blockDim.x + threadIdx.x, nn = (int)Lc.nn;
-    if (i >= 3 * nn) return;
-    const int c = i / nn, n = i - c * nn;
+    if (i >= 3 / COMPS * nn) return;
+    const int c0 = COMPS == 1 ? i / nn : 0, n = i - c0 * nn;
     const int cnx = Lc.nx + 1, cny = Lc.ny + 1;
     const int fny = Lf.ny + 1, fnz = Lf.nz + 1;
     const int cx = n % cnx, cy = (n / cnx) % cny, cz = n / (cnx * cny);
-    const float* __restrict__ a = a1 + (int64_t)c * fnz * fny * cnx + cx;
-    float v = 0.0f;
+    const int64_t n1 = (int64_t)fnz * fny * cnx;
+    const float* __restrict__ a = a1 + c0 * n1 + cx;
+    float v[COMPS];
+#pragma unroll
+    for (int k = 0; k < COMPS; ++k) v[k] = 0.0f;
 #pragma unroll
     for (int iz = 0; iz < WS; ++iz) {
         const int fz = cz * SP + iz - (SP - 1);
         const bool zin = fz >= 0 && fz < fnz;
-        float q[WS];
+        float q[COMPS][WS];
 #pragma unroll
         for (int iy = 0; iy < WS; ++iy) {
             const int fy = cy * SP + iy - (SP - 1);
-            q[iy] = zin && fy >= 0 && fy < fny ? a[(fz * fny + fy) * cnx] : 0.0f;
-        }
-        float t = 0.0f;
+            const bool in = zin && fy >= 0 && fy < fny;
 #pragma unroll
-        for (int iy = 0; iy < WS; ++iy) t = fmaf(hatf(iy, SP), q[iy], t);
-        v = fmaf(hatf(iz, SP), t, v);
+            for (int k = 0; k < COMPS; ++k) q[k][iy] = in ? a[k * n1 + (fz * fny + fy) * cnx] : 0.0f;
+        }
+#pragma unroll
+        for (int k = 0; k < COMPS; ++k) {
+            float t = 0.0f;
+#pragma unroll
+            for (int iy = 0; iy < WS; ++iy) t = fmaf(hatf(iy, SP), q[k][iy], t);
+            v[k] = fmaf(hatf(iz, SP), t, v[k]);
+        }
     }
-    restrict_store32<SP>(Lc, Lf, n, c, cx, cy, cz, v, normalize, rc, x0, w0);
+#pragma unroll
+    for (int k = 0; k < COMPS; ++k)
+        restrict_store32<SP>(Lc, Lf, n, c0 + k, cx, cy, cz, v[k], normalize, rc, x0, w0);
 }
-template <int SP>
+template <int SP, int COMPS>
 __global__ void __launch_bounds__(256) k_restrict_yz32(MgLevel32 Lc, MgLevel32 Lf, const float* __restrict__ a1,
                                                        float* __restrict__ rc, const PcgScalars* S, int normalize,
                                                        float* __restrict__ x0, float w0) {
-    restrict_yz32<SP>(vb_real(), Lc, Lf, a1, rc, S, normalize, x0, w0);
+    restrict_yz32<SP, COMPS>(vb_real(), Lc, Lf, a1, rc, S, normalize, x0, w0);
 }
 
 // The whole 3D window of the fine residual in one pass (levels small enough to sit in L2).
@@ -625,7 +639,8 @@ __global__ void __launch_bounds__(256) k_batch_restrict32(const BatchRestrict* _
         const MgLevel32 Lc = A.Lc, Lf = A.Lf;
         if (Lc.span == 4) {
             if (stage == 0) restrict_x32(vb, Lc, Lf, A.rf, A.a1, A.S);
-            else restrict_yz32<4>(vb, Lc, Lf, A.a1, A.rc, A.S, A.normalize, A.x0, A.w);
+            else if (Lc.nn <= RESTRICT32_LARGE) restrict_yz32<4, 1>(vb, Lc, Lf, A.a1, A.rc, A.S, A.normalize, A.x0, A.w);
+            else restrict_yz32<4, 3>(vb, Lc, Lf, A.a1, A.rc, A.S, A.normalize, A.x0, A.w);
         } else {
             restrict_xyz32<2>(vb, Lc, Lf, A.rf, A.rc, A.S, A.normalize, A.x0, A.w);
         }
@@ -682,7 +697,7 @@ int batch_blocks_restrict(const BatchRestrict& a, int stage) {
     const MgLevel32& Lf = a.Lf;
     if (Lc.span == 4) {
         if (stage == 0) return (int)blocks_for((int64_t)(Lf.nz + 1) * (Lf.ny + 1) * (Lc.nx + 1), 256);
-        return (int)blocks_for(3 * Lc.nn, 256);
+        return (int)blocks_for(Lc.nn <= RESTRICT32_LARGE ? 3 * Lc.nn : Lc.nn, 256);
     }
     return stage == 0 ? (int)blocks_for(3 * Lc.nn, 256) : 0;
 }
@@ -746,7 +761,10 @@ void launch_restrict32(const MgLevel32& Lc, const MgLevel32& Lf, const float* rf
     const int64_t n1 = (int64_t)(Lf.nz + 1) * (Lf.ny + 1) * (Lc.nx + 1);
     if (Lc.span == 4) {
         k_restrict_x32<<<blocks_for(n1, 256), 256, 0, s>>>(Lc, Lf, rf, a1, S);
-        k_restrict_yz32<4><<<blocks_for(3 * Lc.nn, 256), 256, 0, s>>>(Lc, Lf, a1, rc, S, normalize ? 1 : 0, x0, w);
+        if (Lc.nn <= RESTRICT32_LARGE)
+            k_restrict_yz32<4, 1><<<blocks_for(3 * Lc.nn, 256), 256, 0, s>>>(Lc, Lf, a1, rc, S, normalize ? 1 : 0, x0, w);
+        else
+            k_restrict_yz32<4, 3><<<blocks_for(Lc.nn, 256), 256, 0, s>>>(Lc, Lf, a1, rc, S, normalize ? 1 : 0, x0, w);
     } else {
         k_restrict_xyz32<2><<<blocks_for(3 * Lc.nn, 256), 256, 0, s>>>(Lc, Lf, rf, rc, S, normalize ? 1 : 0, x0, w);
     }

@@ -1,6 +1,6 @@
 """The Adapted V-cycle's forms for a level 1 of more than 100,000 nodes -- the first restriction in one pass per axis,
 a node's three components in one thread of the level's prolongation -- against the oracle, bit for bit, on a grid of
-ragged sides (level 1 has 77 x 37 x 39 nodes)."""
+ragged sides (level 1 has 77 x 37 x 39 nodes); and the FP32 cycle's restriction at that size against the FP64 cycle."""
 import numpy as np
 import pytest
 
@@ -24,4 +24,15 @@ def test_adapted_vcycle_large_level_bit_exact_with_oracle():
     L = len(P.levels)
     assert P.kernel_launches() - n0 == 3 + (L - 2) + 1 + (L - 1)
     np.testing.assert_array_equal(z, O.vcycle(r))
+    P.close()
+
+
+def test_fp32_adapted_vcycle_large_level_matches_fp64():
+    import algorithmengineering_altproject_b200 as t3d
+    P = t3d.Problem(143, 301, 150, precision=t3d.T3D_MIXED)
+    rng = np.random.default_rng(29)
+    P.make_diagonal_preconditioner_from_static(rng.uniform(0.05, 1.0, P.ne))
+    r = rng.standard_normal(P.nf).astype(np.float32).astype(np.float64)
+    z = P.vcycle(r)
+    assert np.linalg.norm(P.vcycle32(r) - z) <= 1e-5 * np.linalg.norm(z)
     P.close()
