@@ -36,3 +36,19 @@ def test_fp32_adapted_vcycle_large_level_matches_fp64():
     z = P.vcycle(r)
     assert np.linalg.norm(P.vcycle32(r) - z) <= 1e-5 * np.linalg.norm(z)
     P.close()
+
+
+@pytest.mark.parametrize("dims", [(55, 127, 61), (63, 133, 70), (143, 301, 150)])
+def test_coarse_diagonals_bit_exact_with_oracle(dims):
+    """Level-1 diagonals (8,415, 11,305 and 111,111 nodes) on both sides of the 10,000 nodes from which a thread takes a node's three components."""
+    import algorithmengineering_altproject_b200 as t3d
+    from oracle.bindings import Oracle
+    P = t3d.Problem(*dims)
+    O = Oracle(*dims, red_mode=1, pow_mode=0, vol_mode=0, approx_mode=0)
+    rng = np.random.default_rng(31)
+    E = np.where(rng.random(P.ne) < 0.3, 1e-6, rng.uniform(0.05, 1.0, P.ne))
+    P.make_diagonal_preconditioner_from_static(E)
+    O.mg_build(E)
+    for l in range(len(P.levels)):
+        np.testing.assert_array_equal(P.mg_diag(l), O.mg_diag(l))
+    P.close()
