@@ -472,6 +472,13 @@ int create(int nely, int nelx, int nelz, const t3d_params* prm, const t3d_proble
     }
     CHECK(build_levels(c));
     if (c->mixed) CHECK(build_mixed(c));
+    // device memory of the layout maps and of the staging buffer of host copies, so that reading a result never has to
+    // allocate; the maps themselves are built at their first use.  Free nodes belong to solid elements, so the box of
+    // elements bounds their DOFs, and there are fewer elements than that.
+    c->max_free = (size_t)3 * (nelx + 1) * (nely + 1) * (nelz + 1);
+    CHECK(c->alloc(&c->morton, c->ne));
+    CHECK(c->alloc(&c->free_d, c->max_free));
+    CHECK(c->alloc(&c->stage, c->max_free));
     launch_filter_diag(g, c->solid, c->kf, c->fdiag, c->st);
     CHECK(launch_check("filter set-up"));
     return sync(c);
@@ -496,42 +503,36 @@ static void morton_walk(const Context* c, int x0, int y0, int z0, int h, std::ve
 }
 
 int ensure_morton(Context* c) {
-    if (c->morton) return T3D_OK;
+    if (c->morton_ready) return T3D_OK;
     int h = 1;
     while (h < std::max(c->cub.nelx, std::max(c->cub.nely, c->cub.nelz))) h *= 2;
     c->morton_h.clear();
     c->morton_h.reserve(c->ne);
     morton_walk(c, 0, 0, 0, h, c->morton_h);
-    CHECK(c->alloc(&c->morton, c->ne));
     T3D_CUDA_OK(cudaMemcpyAsync(c->morton, c->morton_h.data(), c->ne * sizeof(int32_t), cudaMemcpyHostToDevice,
                                 c->st));
+    c->morton_ready = true;
     return T3D_OK;
 }
 
 static int ensure_free(Context* c) {
-    if (c->free_d) return T3D_OK;
+    if (c->free_ready) return T3D_OK;
     std::vector<uint8_t> m(c->g.NN);
     T3D_CUDA_OK(cudaMemcpy(m.data(), c->mask0, c->g.NN, cudaMemcpyDeviceToHost));
     c->free_h.clear();
     for (int64_t n = 0; n < c->g.NN; ++n)
         for (int k = 0; k < 3; ++k)
             if (!((m[n] >> k) & 1)) c->free_h.push_back((int32_t)(3 * n + k));
-    CHECK(c->alloc(&c->free_d, c->free_h.size()));
+    if (c->free_h.size() > c->max_free) return set_error(T3D_ERR_CUDA, "free DOFs outside the element box");
     T3D_CUDA_OK(cudaMemcpyAsync(c->free_d, c->free_h.data(), c->free_h.size() * sizeof(int32_t),
                                 cudaMemcpyHostToDevice, c->st));
+    c->free_ready = true;
     return T3D_OK;
-}
-
-// the staging buffer: room for every DOF or element, whichever is more (the maps are built by their users)
-static int ensure_stage(Context* c) {
-    if (c->stage) return T3D_OK;
-    return c->alloc(&c->stage, std::max((size_t)(3 * c->g.NN), (size_t)c->ne));
 }
 
 // host free vector -> device grid vector (fixed DOFs zero)
 static int upload_free(Context* c, const double* h, double* grid) {
     CHECK(ensure_free(c));
-    CHECK(ensure_stage(c));
     const int64_t nf = (int64_t)c->free_h.size();
     T3D_CUDA_OK(cudaMemsetAsync(grid, 0, 3 * c->g.NN * sizeof(double), c->st));
     T3D_CUDA_OK(cudaMemcpyAsync(c->stage, h, nf * sizeof(double), cudaMemcpyHostToDevice, c->st));
@@ -540,7 +541,6 @@ static int upload_free(Context* c, const double* h, double* grid) {
 }
 static int download_free(Context* c, const double* grid, double* h) {
     CHECK(ensure_free(c));
-    CHECK(ensure_stage(c));
     const int64_t nf = (int64_t)c->free_h.size();
     launch_gather_free(nf, c->free_d, grid, c->g.NN, c->stage, c->st);
     CHECK(launch_check("gather_free"));
@@ -549,7 +549,6 @@ static int download_free(Context* c, const double* grid, double* h) {
 }
 static int upload_cells_f64(Context* c, const double* h, double* cells) {
     CHECK(ensure_morton(c));
-    CHECK(ensure_stage(c));
     T3D_CUDA_OK(cudaMemsetAsync(cells, 0, c->g.NE * sizeof(double), c->st));
     T3D_CUDA_OK(cudaMemcpyAsync(c->stage, h, c->ne * sizeof(double), cudaMemcpyHostToDevice, c->st));
     launch_cells_from_morton_f64(c->ne, c->morton, c->stage, cells, c->st);
@@ -557,7 +556,6 @@ static int upload_cells_f64(Context* c, const double* h, double* cells) {
 }
 static int download_cells_f64(Context* c, const double* cells, double* h) {
     CHECK(ensure_morton(c));
-    CHECK(ensure_stage(c));
     launch_cells_to_morton_f64(c->ne, c->morton, cells, c->stage, c->st);
     CHECK(launch_check("cells_to_morton"));
     T3D_CUDA_OK(cudaMemcpyAsync(h, c->stage, c->ne * sizeof(double), cudaMemcpyDeviceToHost, c->st));
@@ -565,7 +563,6 @@ static int download_cells_f64(Context* c, const double* cells, double* h) {
 }
 static int upload_cells_f32(Context* c, const float* h, float* cells) {
     CHECK(ensure_morton(c));
-    CHECK(ensure_stage(c));
     float* st = reinterpret_cast<float*>(c->stage);
     T3D_CUDA_OK(cudaMemsetAsync(cells, 0, c->g.NE * sizeof(float), c->st));
     T3D_CUDA_OK(cudaMemcpyAsync(st, h, c->ne * sizeof(float), cudaMemcpyHostToDevice, c->st));
@@ -574,7 +571,6 @@ static int upload_cells_f32(Context* c, const float* h, float* cells) {
 }
 static int download_cells_f32(Context* c, const float* cells, float* h) {
     CHECK(ensure_morton(c));
-    CHECK(ensure_stage(c));
     float* st = reinterpret_cast<float*>(c->stage);
     launch_cells_to_morton_f32(c->ne, c->morton, cells, st, c->st);
     CHECK(launch_check("cells_to_morton"));

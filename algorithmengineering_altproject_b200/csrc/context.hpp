@@ -96,12 +96,15 @@ struct Context {
     cudaGraphExec_t pcg32_graph = nullptr;
     int64_t pcg32_graph_launches = 0;
     int last_outer = 0;
-    // lazily built maps between the reference's layouts and the grid
+    // maps between the reference's layouts and the grid: allocated at creation, built at their first use
     int32_t* morton = nullptr;          // [ne] cell index of the k-th element in Morton order
     std::vector<int32_t> morton_h;
-    int32_t* free_d = nullptr;
+    bool morton_ready = false;
+    int32_t* free_d = nullptr;          // [max_free] free DOFs, ascending
     std::vector<int32_t> free_h;
-    double* stage = nullptr;            // staging buffer for host<->device conversions
+    bool free_ready = false;
+    size_t max_free = 0;                // DOFs of the element box
+    double* stage = nullptr;            // [max_free] staging buffer for host<->device conversions
     // pinned host mirror of small device state
     PcgScalars* S_h = nullptr;
     OcState* OC_h = nullptr;
