@@ -271,7 +271,7 @@ static int batch_lists(Batch* B) {
             const float* src = B->standard ? (l == 0 ? c->Ap32 : c->vtmp32[l]) : (l == 0 ? c->r32 : c->lv32[l].r);
             // the Standard cycle starts the coarse level in the same kernel (the coarsest level is solved instead)
             float* x0 = B->standard && l + 2 < c->nlev ? c->lv32[l + 1].x : nullptr;
-            return BatchRestrict{c->lv32[l + 1], c->lv32[l], src, c->ra1_32[l], c->lv32[l + 1].r, c->S32, norm, x0,
+            return BatchRestrict{c->lv32[l + 1], c->lv32[l], src, c->ra1_32, c->lv32[l + 1].r, c->S32, norm, x0,
                                  c->prm.mg_standard_weight};
         };
         CHECK(list(&B->rs0[l], below, rs, [](const BatchRestrict& a) { return batch_blocks_restrict(a, 0); }));

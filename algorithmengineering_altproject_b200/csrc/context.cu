@@ -141,7 +141,8 @@ static int build_levels(Context* c) {
     }
     for (int l = 0; l + 1 < c->nlev; ++l) {
         const MgLevel &Lf = c->lv[l], &Lc = c->lv[l + 1];
-        CHECK(c->alloc(&c->ra1[l], (size_t)3 * (Lf.nz + 1) * (Lf.ny + 1) * (Lc.nx + 1)));
+        if (Lc.span != 4) continue;   // a span-2 restriction is one pass; only the first transition can have span 4
+        CHECK(c->alloc(&c->ra1, (size_t)3 * (Lf.nz + 1) * (Lf.ny + 1) * (Lc.nx + 1)));
         if (restrict_by_axes(Lc)) CHECK(c->alloc(&c->ra2, (size_t)3 * (Lf.nz + 1) * (Lc.ny + 1) * (Lc.nx + 1)));
     }
     T3D_CUDA_OK(mg_kernel_attributes());
@@ -203,7 +204,7 @@ static int build_mixed(Context* c) {
     }
     for (int l = 0; l + 1 < c->nlev; ++l) {
         const MgLevel &Lf = c->lv[l], &Lc = c->lv[l + 1];
-        CHECK(c->alloc(&c->ra1_32[l], (size_t)3 * (Lf.nz + 1) * (Lf.ny + 1) * (Lc.nx + 1)));
+        if (Lc.span == 4) CHECK(c->alloc(&c->ra1_32, (size_t)3 * (Lf.nz + 1) * (Lf.ny + 1) * (Lc.nx + 1)));
     }
     if (c->standard) {
         CHECK(c->alloc(&c->E_mg32, g.NEp));
@@ -406,7 +407,6 @@ int create(int nely, int nelx, int nelz, const t3d_params* prm, const t3d_proble
     CHECK(c->alloc(&c->E, g.NE));
     CHECK(c->alloc(&c->ce, g.NE));
     CHECK(c->alloc(&c->x, g.NE));
-    CHECK(c->alloc(&c->xnew, g.NE));
     CHECK(c->alloc(&c->dc, g.NE));
     CHECK(c->alloc(&c->xdc, g.NE));
     CHECK(c->alloc(&c->dcf, g.NE));
@@ -452,7 +452,7 @@ int create(int nely, int nelx, int nelz, const t3d_params* prm, const t3d_proble
     // zero every array once: ghost cells and non-solid cells stay exactly zero from here on
     T3D_CUDA_OK(cudaMemsetAsync(c->E, 0, g.NE * sizeof(double), c->st));
     T3D_CUDA_OK(cudaMemsetAsync(c->ce, 0, g.NE * sizeof(double), c->st));
-    for (float* v : {c->x, c->xnew, c->dc, c->xdc, c->dcf})
+    for (float* v : {c->x, c->dc, c->xdc, c->dcf})
         T3D_CUDA_OK(cudaMemsetAsync(v, 0, g.NE * sizeof(float), c->st));
     for (double* v : {c->b, c->u, c->r, c->z, c->p, c->Ap})
         T3D_CUDA_OK(cudaMemsetAsync(v, 0, 3 * g.NN * sizeof(double), c->st));
@@ -690,7 +690,7 @@ static void vcycle_standard(Context* c, const double* r, double* z, PcgScalars* 
     for (int l = 0; l + 1 < L; ++l) {
         const MgLevel &Lf = c->lv[l], &Lc = c->lv[l + 1];
         if (l > 0) launch_level_op(Lf, c->KelT[l], Lf.x, Lf.r, c->vtmp[l], false, w, S, c->st);
-        launch_restrict(Lc, Lf, l == 0 ? c->Ap : c->vtmp[l], Lc.r, c->ra1[l], c->ra2, S, c->st, false,
+        launch_restrict(Lc, Lf, l == 0 ? c->Ap : c->vtmp[l], Lc.r, c->ra1, c->ra2, S, c->st, false,
                         l + 2 < L ? Lc.x : nullptr, w);
     }
     launch_coarse_solve(c->lv[L - 1], c->Xc, c->Nc, c->chol_status, S, c->st);
@@ -715,7 +715,7 @@ static void vcycle(Context* c, const double* r, double* z, PcgScalars* S, RedSlo
     const int L = c->nlev, tail = adapted_tail_first(c->lv, L, c->Nc), down = std::min(tail, L - 1);
     c->launches += vcycle_launches(c);
     for (int l = 0; l < down; ++l)
-        launch_restrict(c->lv[l + 1], c->lv[l], l == 0 ? r : c->lv[l].r, c->lv[l + 1].r, c->ra1[l], c->ra2, S, c->st);
+        launch_restrict(c->lv[l + 1], c->lv[l], l == 0 ? r : c->lv[l].r, c->lv[l + 1].r, c->ra1, c->ra2, S, c->st);
     if (tail < L)
         launch_adapted_tail(c->lv, L, tail, c->Xc, c->Nc, c->chol_status, (double)c->prm.mg_weight, S, c->st);
     else
@@ -817,7 +817,7 @@ static void vcycle32_standard(Context* c, const float* r, float* z, PcgScalars* 
     for (int l = 0; l + 1 < L; ++l) {
         const MgLevel32 &Lf = c->lv32[l], &Lc = c->lv32[l + 1];
         if (l > 0) launch_level_op32(Lf, c->Kel32[l], Lf.x, Lf.r, c->vtmp32[l], false, w, S, c->st);
-        launch_restrict32(Lc, Lf, l == 0 ? c->Ap32 : c->vtmp32[l], Lc.r, c->ra1_32[l], S, c->st, false,
+        launch_restrict32(Lc, Lf, l == 0 ? c->Ap32 : c->vtmp32[l], Lc.r, c->ra1_32, S, c->st, false,
                           l + 2 < L ? Lc.x : nullptr, w);
         c->launches += (l > 0) + (Lc.span == 4 ? 2 : 1);
     }
@@ -856,7 +856,7 @@ static void vcycle32(Context* c, const float* r, float* z, PcgScalars* S, RedSlo
     for (int l = 0; l + 1 < L; ++l) c->launches += c->lv32[l + 1].span == 2 ? 2 : 3;
     c->launches += 1;
     for (int l = 0; l + 1 < L; ++l)
-        launch_restrict32(c->lv32[l + 1], c->lv32[l], l == 0 ? r : c->lv32[l].r, c->lv32[l + 1].r, c->ra1_32[l], S,
+        launch_restrict32(c->lv32[l + 1], c->lv32[l], l == 0 ? r : c->lv32[l].r, c->lv32[l + 1].r, c->ra1_32, S,
                           c->st);
     launch_coarse_solve32(c->lv32[L - 1], c->Xc, c->Nc, c->chol_status, S, c->st);
     for (int l = L - 2; l >= 1; --l)
@@ -1655,9 +1655,9 @@ int t3d_export_stl(t3d_context* ctx, const float* xphys, float iso, const char* 
     if (!path) return t3d::set_error(T3D_ERR_INVALID, "null path");
     const t3d::Grid& g = ctx->g;
     const float* dens = ctx->x;
-    if (xphys) {   // densities given in the reference's element order: staged into xnew (cells)
-        CHECK(t3d::upload_cells_f32(ctx, xphys, ctx->xnew));
-        dens = ctx->xnew;
+    if (xphys) {   // densities given in the reference's element order: in dcf, whose values live within one call only
+        CHECK(t3d::upload_cells_f32(ctx, xphys, ctx->dcf));
+        dens = ctx->dcf;
     }
     const int nb = t3d::stl_chunks(g);
     unsigned* bsum = nullptr;

@@ -46,7 +46,7 @@ struct Context {
     uint8_t* solid = nullptr;   // cells
     uint8_t* mask0 = nullptr;   // nodes
     double *E = nullptr, *ce = nullptr;                       // cells
-    float *x = nullptr, *xnew = nullptr, *dc = nullptr, *xdc = nullptr, *dcf = nullptr;   // cells
+    float *x = nullptr, *dc = nullptr, *xdc = nullptr, *dcf = nullptr;   // cells
     double *b = nullptr, *u = nullptr, *r = nullptr, *z = nullptr, *p = nullptr, *Ap = nullptr;  // 3 NN
     PcgScalars* S = nullptr;
     FilterScalars* FS = nullptr;
@@ -71,7 +71,7 @@ struct Context {
     double* Kd = nullptr;       // [KE_MAX_DISTINCT]
     RedSlot slot[4]{};
     double *Kce = nullptr, *Kc = nullptr, *LT = nullptr, *Lrow = nullptr, *Xc = nullptr;
-    double* ra1[8]{};           // x-pass buffer of the separable restriction per level transition
+    double* ra1 = nullptr;      // x-pass buffer of a span-4 first transition's separable restriction
     double* ra2 = nullptr;      // y-pass buffer of a large first transition (restrict_by_axes)
     int* chol_status = nullptr;
     double *frhs = nullptr, *fx = nullptr, *fr = nullptr, *fz = nullptr, *fp = nullptr, *fAp = nullptr,
@@ -86,7 +86,7 @@ struct Context {
     float* E32 = nullptr;
     float *r32 = nullptr, *d32 = nullptr, *z32 = nullptr, *p32 = nullptr, *Ap32 = nullptr;
     MgLevel32 lv32[8]{};
-    float* ra1_32[8]{};         // x-pass buffer of the FP32 restriction (its y and z passes are fused)
+    float* ra1_32 = nullptr;    // the same in FP32
     // the Standard V-cycle in FP32: element-matrix images and scratch per coarse level, level-0 moduli image
     float* Kel32[8]{};
     float* vtmp32[8]{};
