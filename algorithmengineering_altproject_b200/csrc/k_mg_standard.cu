@@ -394,10 +394,8 @@ __global__ void k_to_coarse_layout(MgLevel L, const double* __restrict__ Kel, do
     Kce[(int64_t)cel * 576 + k] = Kel[t];
 }
 
-// element-major -> entry-major (dst[k * ne + e] = src[e * 576 + k]) through 32 x 32 shared-memory tiles, with
-// the FP32 image written instead when B is float
-template <class B>
-__global__ void k_kel_transpose(int64_t ne, const double* __restrict__ src, B* __restrict__ dst) {
+// element-major -> entry-major (dst[k * ne + e] = src[e * 576 + k]) through 32 x 32 shared-memory tiles
+__global__ void k_kel_transpose(int64_t ne, const double* __restrict__ src, double* __restrict__ dst) {
     __shared__ double tile[32][33];
     const int64_t e0 = (int64_t)blockIdx.x * 32;
     const int k0 = blockIdx.y * 32;
@@ -410,7 +408,7 @@ __global__ void k_kel_transpose(int64_t ne, const double* __restrict__ src, B* _
     for (int j = threadIdx.y; j < 32; j += blockDim.y) {   // rows = entries, columns = elements (coalesced in e)
         const int k = k0 + j;
         const int64_t e = e0 + threadIdx.x;
-        if (e < ne && k < 576) dst[(int64_t)k * ne + e] = (B)tile[threadIdx.x][j];
+        if (e < ne && k < 576) dst[(int64_t)k * ne + e] = tile[threadIdx.x][j];
     }
 }
 
@@ -419,12 +417,8 @@ inline unsigned blocks_of(int64_t n, int t) { return (unsigned)((n + t - 1) / t)
 }  // namespace
 
 void launch_kel_transpose(int64_t ne, const double* Kel, double* KelT, cudaStream_t s) {
-    k_kel_transpose<double><<<dim3((unsigned)((ne + 31) / 32), 18), dim3(32, 8), 0, s>>>(ne, Kel, KelT);
+    k_kel_transpose<<<dim3((unsigned)((ne + 31) / 32), 18), dim3(32, 8), 0, s>>>(ne, Kel, KelT);
 }
-void launch_kel_transpose32(int64_t ne, const double* Kel, float* KelT32, cudaStream_t s) {
-    k_kel_transpose<float><<<dim3((unsigned)((ne + 31) / 32), 18), dim3(32, 8), 0, s>>>(ne, Kel, KelT32);
-}
-
 void galerkin_positions(int s, const double* Ke, double* G) {
     for (int k = 0; k < s; ++k)
         for (int j = 0; j < s; ++j)

@@ -42,13 +42,15 @@ __device__ __forceinline__ float lane_of(const V& v, int k) {
     return reinterpret_cast<const float*>(&v)[k];
 }
 
-// x = w r / D on the pitched finest level: 4 consecutive row entries per thread (16-byte loads and stores of the
-// pitched vectors; the row's pads past x = nx stay zero).  Same arithmetic per DOF as the generic loop.
-__device__ __forceinline__ void jacobi_init0_32(VB vb, const MgLevel32& L, const float* __restrict__ r,
-                                               float* __restrict__ x, float w) {
+// The finest level's steps of their own: the start, and where the level-0 products are not fused (no modal TMA form) the
+// residual and the correction.  Its vectors are pitched, with the pads past x = nx zero.
+// x = w r / D: 4 consecutive row entries per thread (16-byte loads and stores)
+__global__ void k_jacobi_init32(MgLevel32 L, const float* __restrict__ r, float* __restrict__ x, float w,
+                                const PcgScalars* S) {
+    if (S->done) return;
     const int fnx = L.nx + 1, q4 = L.pitch >> 2;
     const int rows = (L.ny + 1) * (L.nz + 1), per_c = rows * q4;   // 3 per_c < 2^31: the grids' DOFs fit 32 bits
-    for (int t = vb.b * blockDim.x + threadIdx.x; t < 3 * per_c; t += vb.n * blockDim.x) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 3 * per_c; t += gridDim.x * blockDim.x) {
         const int c = t / per_c;
         const int rt = t - c * per_c, row = rt / q4;
         const int x0 = 4 * (rt - row * q4);
@@ -65,6 +67,34 @@ __device__ __forceinline__ void jacobi_init0_32(VB vb, const MgLevel32& L, const
     }
 }
 
+// kx <- r - kx
+__global__ void k_residual32(MgLevel32 L, const float* __restrict__ r, float* __restrict__ kx, const PcgScalars* S) {
+    if (S->done) return;
+    for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < L.nn; n += (int64_t)gridDim.x * blockDim.x) {
+        const int m = L.mask[n];
+        const int64_t v = vidx(L, n);
+        for (int c = 0; c < 3; ++c) {
+            const int64_t i = c * L.cs + v;
+            kx[i] = ((m >> c) & 1) ? 0.0f : r[i] - kx[i];
+        }
+    }
+}
+
+// x += w (r - kx) / D
+__global__ void k_jacobi_correct32(MgLevel32 L, const float* __restrict__ r, const float* __restrict__ kx,
+                                   float* __restrict__ x, float w, const PcgScalars* S) {
+    if (S->done) return;
+    for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < L.nn; n += (int64_t)gridDim.x * blockDim.x) {
+        const int m = L.mask[n];
+        const int64_t v = vidx(L, n);
+        for (int c = 0; c < 3; ++c) {
+            const int64_t i = c * L.cs + v;
+            x[i] = ((m >> c) & 1) ? 0.0f : x[i] + (w * (r[i] - kx[i])) * L.diag[i];
+        }
+    }
+}
+
+// (kernel bodies that the batched launches below share take the logical block VB)
 // xo = xi + P xc on the pitched finest level.  A thread takes a run of SP consecutive fine nodes of one row that
 // share one coarse cell (fine x = SP j + k; the row's last node, x = nx, clamped to the last coarse cell, is a run
 // of its own): the cell's 8 corners are loaded once for the run and its nodes move as one SP-wide vector.
@@ -144,68 +174,6 @@ __device__ __forceinline__ void prolong_add0_32(VB vb, const MgLevel32& Lc, cons
             *reinterpret_cast<V*>(xo + c * Lf.cs + rb) = o;
         }
     }
-}
-
-// x = w r / D
-// (kernel bodies take the logical block VB, so that the batched launches below run them unchanged)
-__device__ __forceinline__ void jacobi_init32(VB vb, const MgLevel32& L, const float* __restrict__ r,
-                                              float* __restrict__ x, float w, const PcgScalars* S) {
-    if (S->done) return;
-    if (L.pitch != L.nx + 1) {   // the pitched finest level
-        jacobi_init0_32(vb, L, r, x, w);
-        return;
-    }
-    for (int64_t n = (int64_t)vb.b * blockDim.x + threadIdx.x; n < L.nn; n += (int64_t)vb.n * blockDim.x) {
-        const int m = L.mask[n];
-        const int64_t v = vidx(L, n);
-        for (int c = 0; c < 3; ++c) {
-            const int64_t i = c * L.cs + v;
-            x[i] = ((m >> c) & 1) ? 0.0f : (w * r[i]) * L.diag[i];
-        }
-    }
-}
-
-__global__ void k_jacobi_init32(MgLevel32 L, const float* __restrict__ r, float* __restrict__ x, float w,
-                                const PcgScalars* S) {
-    jacobi_init32(vb_real(), L, r, x, w, S);
-}
-
-// kx <- r - kx
-__device__ __forceinline__ void residual32(VB vb, const MgLevel32& L, const float* __restrict__ r,
-                                           float* __restrict__ kx, const PcgScalars* S) {
-    if (S->done) return;
-    for (int64_t n = (int64_t)vb.b * blockDim.x + threadIdx.x; n < L.nn; n += (int64_t)vb.n * blockDim.x) {
-        const int m = L.mask[n];
-        const int64_t v = vidx(L, n);
-        for (int c = 0; c < 3; ++c) {
-            const int64_t i = c * L.cs + v;
-            kx[i] = ((m >> c) & 1) ? 0.0f : r[i] - kx[i];
-        }
-    }
-}
-
-__global__ void k_residual32(MgLevel32 L, const float* __restrict__ r, float* __restrict__ kx, const PcgScalars* S) {
-    residual32(vb_real(), L, r, kx, S);
-}
-
-// x += w (r - kx) / D
-__device__ __forceinline__ void jacobi_correct32(VB vb, const MgLevel32& L, const float* __restrict__ r,
-                                                 const float* __restrict__ kx, float* __restrict__ x, float w,
-                                                 const PcgScalars* S) {
-    if (S->done) return;
-    for (int64_t n = (int64_t)vb.b * blockDim.x + threadIdx.x; n < L.nn; n += (int64_t)vb.n * blockDim.x) {
-        const int m = L.mask[n];
-        const int64_t v = vidx(L, n);
-        for (int c = 0; c < 3; ++c) {
-            const int64_t i = c * L.cs + v;
-            x[i] = ((m >> c) & 1) ? 0.0f : x[i] + (w * (r[i] - kx[i])) * L.diag[i];
-        }
-    }
-}
-
-__global__ void k_jacobi_correct32(MgLevel32 L, const float* __restrict__ r, const float* __restrict__ kx,
-                                   float* __restrict__ x, float w, const PcgScalars* S) {
-    jacobi_correct32(vb_real(), L, r, kx, x, w, S);
 }
 
 // xo = xi + P xc (trilinear from the coarse cell floor(f/s), clamped to the last cell), fixed DOFs 0; xo may be xi

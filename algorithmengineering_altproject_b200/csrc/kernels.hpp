@@ -160,7 +160,6 @@ void launch_coarse_solve(const MgLevel& L, const double* X, int N, const int* st
 // level with ne elements at kel_index(e, k, ne) = k * ne + e.
 __host__ __device__ inline int64_t kel_index(int64_t e, int k, int64_t ne) { return (int64_t)k * ne + e; }
 void launch_kel_transpose(int64_t ne, const double* Kel, double* KelT, cudaStream_t s);
-void launch_kel_transpose32(int64_t ne, const double* Kel, float* KelT32, cudaStream_t s);
 // G[pos][576] = W_pos^T Ke W_pos for the s^3 child positions of a span-s coarse element (host)
 void galerkin_positions(int s, const double* Ke, double* G);
 void launch_galerkin_fine(const Grid& g, const MgLevel& L1, const double* E, const uint8_t* mask0, const double* Gpos,
