@@ -248,7 +248,7 @@ class Oracle(_Common):
         return cls._lib
 
     def __init__(self, nely, nelx, nelz, emin=None, max_levels=5, pow_mode=0, vol_mode=0, approx_mode=0, red_mode=0,
-                 penal=None, coarse_full=0, voxel_model=None):
+                 penal=None, coarse_full=0, voxel_model=None, nondyadic=1):
         """voxel_model: an external (TopVoxel) model from `voxel_model_from_rows`, else the cantilever."""
         L = self.lib()
         p = OrcParams()
@@ -258,6 +258,7 @@ class Oracle(_Common):
         if penal is not None:
             p.penal = penal
         p.mg_max_levels = max_levels
+        p.mg_nondyadic = nondyadic
         p.pow_mode = pow_mode
         p.vol_mode = vol_mode
         p.approx_mode = approx_mode
