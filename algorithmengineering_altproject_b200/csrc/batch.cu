@@ -807,9 +807,7 @@ int t3d_batch_member(t3d_batch* b, int i, t3d_context** out) {
     return T3D_OK;
 }
 
-// One member after another: initialisations run from parallel host threads (each a first solve that also
-// captures the member's PCG graph) gave, in about one run in three of 48 members, an exactly zero solid-domain
-// compliance for one small member; one at a time they never did.  The cause was not found.
+// One member after another, each on its own stream (a first solve also captures the member's PCG graph).
 int t3d_batch_design_init(t3d_batch* b, const float* V0, double* c_solid) {
     if (!b || !V0) return t3d::set_error(T3D_ERR_INVALID, "null argument");
     if (cudaSetDevice(b->dev) != cudaSuccess) return t3d::set_error(T3D_ERR_CUDA, "cudaSetDevice failed");

@@ -879,7 +879,7 @@ void launch_coarse_inverse(const double* LT, const double* Lrow, int N, const in
 void launch_coarse_solve(const MgLevel& L, const double* X, int N, const int* status, const PcgScalars* S,
                          cudaStream_t s) {
     const unsigned blocks = N > 0 ? blocks_for(N, 32) : blocks_for(3 * L.nn, CS_THREADS);
-    const size_t smem = (size_t)(std::max(N, 0) + 32 * CS_ROWS) * sizeof(double);   // N <= 1000: at most 72 KB
+    const size_t smem = (size_t)(std::max(N, 0) + 32 * CS_ROWS) * sizeof(double);   // N <= 1000: at most 41 KB
     k_coarse_solve<<<blocks, CS_THREADS, smem, s>>>(L, X, N, status, S);
 }
 cudaError_t mg_kernel_attributes() {

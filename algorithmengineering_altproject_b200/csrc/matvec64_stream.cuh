@@ -10,9 +10,9 @@
 // Streaming: a CTA of BX x BY threads (one element column each) owns a (BX-1) x (BY-1) tile of node
 // columns and marches up a slab of node planes; node planes come through a 3-slot cp.async ring in
 // shared memory (the plane below stays in the ring while the plane above arrives).  Per element layer
-// the chains' results for the bottom and top corners go to shared memory; each owned node folds its 4
-// same-layer elements in colour order and carries the other layer's part to the next plane (a partial
-// sum when that layer comes first in the node's colour order, the 4 raw triples otherwise).
+// the chains' results go to shared memory, the top corners' in one of two slots by the layer's parity, so that
+// when the layer above is done each owned node of the plane between folds its 8 elements in colour order (the
+// four of the even layer first).
 // Coefficients: a DFMA whose coefficient is a constant-bank operand issues at about half the rate of
 // one with register operands only, and a shared-memory broadcast of FP64 coefficients costs more than
 // the DFMAs it feeds.  The built-in Ke has only KE_ND distinct magnitudes (ke_pattern.inc), so for it
@@ -20,11 +20,10 @@
 // modifier); the 24 rows of a column run in ke_row_order so that consecutive DFMAs share a coefficient
 // register.  Any other Ke (t3d_set_ke) is passed by value and read from the constant bank.
 // p.Ap is not fused: the caller folds it in the canonical order.
-// What bounds it: the chains are 576 DFMAs a thread and layer, 1.3 ms at 256x512x256 with the tile halo; the rest of a
-// layer used to be as many instructions again (index divisions in the loads, corner and side arithmetic in the fold:
-// FP64 pipe 49 % busy, issue slots 49 %), which did not overlap them.  With the loads' places fixed per thread and the
-// fold's order reduced to three parity bits the launch takes 2.33 ms instead of 2.81 (96x192x96: 0.183 -> 0.155 with
-// its dot, 48x96x48 44 -> 36 us).
+// What bounds it: the chains are 576 DFMAs a thread and layer, 1.3 ms at 256x512x256 with the tile halo, and the rest of a
+// layer does not overlap them.  Hence the loads' places fixed per thread and the fold's order reduced to three parity
+// bits: with index divisions in the loads and corner and side arithmetic in the fold, which were as many instructions as
+// the chains, the launch took 2.81 ms, now 2.33 (96x192x96 with its dot 0.183, 0.155; 48x96x48 44 us, 36).
 // One source file per MODE instantiates the kernel (k_matvec64_stream.cu, k_matvec64_residual.cu, k_matvec64_correct.cu):
 // the pattern's unrolled chains take the compiler two minutes each, and the files build side by side.
 #pragma once
