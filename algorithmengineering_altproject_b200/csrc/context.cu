@@ -476,9 +476,9 @@ int create(int nely, int nelx, int nelz, const t3d_params* prm, const t3d_proble
     // allocate; the maps themselves are built at their first use.  Free nodes belong to solid elements, so the box of
     // elements bounds their DOFs, and there are fewer elements than that.
     c->max_free = (size_t)3 * (nelx + 1) * (nely + 1) * (nelz + 1);
-    CHECK(c->alloc(&c->morton, c->ne));
-    CHECK(c->alloc(&c->free_d, c->max_free));
-    CHECK(c->alloc(&c->stage, c->max_free));
+    CHECK(c->alloc(&c->stage, c->max_free + (c->max_free + 1) / 2 + (c->ne + 1) / 2));   // one block, in this order
+    c->free_d = reinterpret_cast<int32_t*>(c->stage + c->max_free);
+    c->morton = reinterpret_cast<int32_t*>(c->stage + c->max_free + (c->max_free + 1) / 2);
     launch_filter_diag(g, c->solid, c->kf, c->fdiag, c->st);
     CHECK(launch_check("filter set-up"));
     return sync(c);
